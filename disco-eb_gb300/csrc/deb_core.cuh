@@ -298,7 +298,8 @@ struct Grp {
   HD bool lead() const { return lane == 0; }
   HD void sync() const {
 #ifdef __CUDA_ARCH__
-    if (G > 1) __syncwarp();
+    if (G > 32) __syncthreads();
+    else if (G > 1) __syncwarp();
 #endif
   }
   HD double sum(double x) const {

@@ -17,7 +17,7 @@ struct deb_plan {
   // lane mode
   int lane_blocks, lane_slots;
   // warp mode
-  int warp_block_warps, warp_blocks, warp_smem, warp_k_global, warp_per_sm;
+  int block_warps, warp_blocks, warp_smem, warp_k_global, warp_per_sm;
   // grouped plans (deb_plan_create_grouped): modes per group, warps in flight
   int group_size, group_warps;
   long warp_smem_bytes;

@@ -23,6 +23,7 @@
 #include <cmath>
 #include <mutex>
 
+#include "deb_block.cuh"
 #include "deb_core.cuh"
 #include "deb_internal.h"
 #include "discoeb_gb300.h"
@@ -207,6 +208,61 @@ __global__ void __launch_bounds__(32, DEB_FWD_MIN_WARPS_PER_SM) forward_warp_ker
   }
 }
 
+// One block of NW warps per mode (deb_block.cuh): the structured solver's
+// kernel.  Four warps fill an SM's FP64 pipe (19 cycles per instruction; one
+// warp gets at most one per 64), four blocks per SM hide its latencies at 128
+// registers a thread.
+template <int NW>
+__global__ void __launch_bounds__(32 * NW, 4) forward_block_kernel(KParams P) {
+  extern __shared__ double smem[];
+  __shared__ __align__(16) unsigned char raw[sizeof(deb::BlkS)];   // no constructor runs
+  deb::BlkS& S = *reinterpret_cast<deb::BlkS*>(raw);
+  const int tid = threadIdx.x;
+  const int nq = P.D.nq;
+  double* const slot = smem + 21 * nq;
+  deb::WS<32> w;
+  w.p = P.smem ? slot : P.ws + (long)blockIdx.x * P.slot_len;
+  w.n = P.D.n;
+  w.misc0 = deb::V_K0 * P.D.n;
+  w.kp = (P.smem && P.kws) ? P.kws + (long)blockIdx.x * deb::stage_len(P.D) : w.p + deb::hot_len(P.D);
+  w.dp = nullptr;
+  deb::Blk<NW> B{S, w, smem, P.D, c_rodas, tid, tid >> 5, tid & 31};
+  B.init_tables(c_tab);
+  for (;;) {
+    if (tid == 0) S.q = atomicAdd(P.queue, 1);
+    __syncthreads();
+    const int q = S.q;
+    if (q >= P.nmode * P.nset) break;
+    const double* tau_out = nullptr;
+    double* yout = nullptr;
+    int m = 0;
+    {
+      deb::Cosmo c;
+      deb::ModeConst mc;
+      deb::Run run;
+      const bool ok = prepare_mode(P, q, c, mc, tau_out, yout, run, m, tid, 32 * NW);
+      __syncthreads();   // S.q read by every thread
+      if (!ok) continue;
+      // rounded as the warp kernel rounds it (grhog + grhor Neff in one operation)
+      mc.grr = __fma_rn(mc.grhor, mc.Neff, mc.grhog);
+      if (tid == 0) { S.c = c; S.m = mc; S.r = run; }
+    }
+    __syncthreads();
+    B.solve(P.ctl, tau_out, yout);
+    if (tid == 0) {
+      const deb::Run& run = S.r;
+      P.status[m] = run.status;
+      if (P.steps) { P.steps[2 * m] = run.acc; P.steps[2 * m + 1] = run.rej; }
+      if (P.ctl.record && P.nrec) P.nrec[m] = run.status == deb::ST_OK ? run.acc : 0;
+      if (P.ctl.record && P.ckstride) P.ckstride[m] = run.ck_stride;
+    }
+    __syncthreads();
+  }
+}
+constexpr int kBlockWarps = 4;
+inline long block_extra_bytes(const deb::Dims& D) { return 21L * D.nq * (long)sizeof(double); }
+inline long block_static_bytes() { return (long)sizeof(deb::BlkS); }
+
 // Groups of B consecutive modes sharing one step sequence (the reference's
 // batched variant): one warp per group, taken from the queue; the group's B
 // slots live in global memory and the warp steps its modes one after the
@@ -322,6 +378,8 @@ unsigned long long g_consts_ctx[64] = {0};
 unsigned long long g_attr_ctx[64] = {0};
 // largest dynamic shared memory size set on forward_warp_kernel, per device
 long g_warp_smem_attr[64] = {0};
+unsigned long long g_block_attr_ctx[64] = {0};
+long g_block_smem_attr[64] = {0};
 
 int upload_constants() {
   int dev = 0;
@@ -348,16 +406,23 @@ int upload_constants() {
 // Raise forward_warp_kernel's dynamic shared memory limit to at least
 // `bytes` in the current context (only ever raised, so that plans made
 // earlier with a larger slot stay launchable).
-int ensure_warp_smem(int dev, long bytes) {
+template <class Kernel>
+int ensure_smem(Kernel* kernel, unsigned long long* attr_ctx, long* attr, int dev, long bytes) {
   const unsigned long long ctx = deb_internal::current_ctx_id();
   std::lock_guard<std::mutex> lock(g_state_mu);
-  const bool known = dev >= 0 && dev < 64 && ctx != 0 && g_attr_ctx[dev] == ctx;
-  if (known && g_warp_smem_attr[dev] >= bytes) return DEB_OK;
-  const long want = known && g_warp_smem_attr[dev] > bytes ? g_warp_smem_attr[dev] : bytes;
-  if (cudaFuncSetAttribute(forward_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want) != cudaSuccess)
+  const bool known = dev >= 0 && dev < 64 && ctx != 0 && attr_ctx[dev] == ctx;
+  if (known && attr[dev] >= bytes) return DEB_OK;
+  const long want = known && attr[dev] > bytes ? attr[dev] : bytes;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want) != cudaSuccess)
     return DEB_ERR_CUDA;
-  if (dev >= 0 && dev < 64) { g_attr_ctx[dev] = ctx; g_warp_smem_attr[dev] = want; }
+  if (dev >= 0 && dev < 64) { attr_ctx[dev] = ctx; attr[dev] = want; }
   return DEB_OK;
+}
+int ensure_warp_smem(int dev, long bytes) {
+  return ensure_smem(forward_warp_kernel, g_attr_ctx, g_warp_smem_attr, dev, bytes);
+}
+int ensure_block_smem(int dev, long bytes) {
+  return ensure_smem(forward_block_kernel<kBlockWarps>, g_block_attr_ctx, g_block_smem_attr, dev, bytes);
 }
 
 }  // namespace
@@ -439,10 +504,16 @@ int deb_plan_create_ex(const deb_dims* dims, int max_modes, const deb_launch_cfg
     // a mode's whole slot in shared memory when 2 modes fit per SM, else only
     // the hot part (vectors before k1 + MISC) with k1..k8 in global memory
     // (L2-resident, lane-strided coalesced access)
-    const long full_bytes = p->slot_len * 8, hot_bytes = deb::hot_len(p->D) * 8;
+    // the structured solver runs a block of kBlockWarps warps per mode
+    // (up to 32 momentum bins: its sums over the bins take one lane per bin)
+    p->block_warps = p->dense || p->D.nq > 32 ? 0 : kBlockWarps;
+    const long extra = p->block_warps ? block_extra_bytes(p->D) : 0;       // dynamic, beside the slot
+    const long fixed = p->block_warps ? block_static_bytes() : 0;
+    smem_optin -= (int)fixed;
+    const long full_bytes = p->slot_len * 8 + extra, hot_bytes = deb::hot_len(p->D) * 8 + extra;
     const long sm_bytes = 228L * 1024;
     long smem_bytes;
-    const bool full_fits = sm_bytes / (full_bytes + 1024) >= 2 && full_bytes <= smem_optin;
+    const bool full_fits = sm_bytes / (full_bytes + fixed + 1024) >= 2 && full_bytes <= smem_optin;
     bool k_global;
     if (stage_where == DEB_STAGE_SHARED) {
       if (full_bytes > smem_optin) { delete p; return DEB_ERR_INVALID; }
@@ -456,18 +527,20 @@ int deb_plan_create_ex(const deb_dims* dims, int max_modes, const deb_launch_cfg
     p->warp_k_global = k_global ? 1 : 0;
     p->warp_smem = smem_bytes <= smem_optin && stage_where != DEB_STAGE_ALL_GLOBAL;
     if (!p->warp_smem) p->warp_k_global = 0;
-    p->warp_block_warps = 1;
     // blocks (= modes in flight) per SM limited by shared memory, by
     // registers (the kernel's own occupancy without shared memory: 8 one-warp
     // blocks at 255 registers per thread) and by the caller's cap
     int per_sm = kMaxWarpBlocksPerSM;
     {
       int occ = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, forward_warp_kernel, 32, 0) == cudaSuccess && occ > 0)
-        per_sm = occ;
+      const cudaError_t e =
+          p->block_warps
+              ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, forward_block_kernel<kBlockWarps>, 32 * kBlockWarps, extra)
+              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, forward_warp_kernel, 32, 0);
+      if (e == cudaSuccess && occ > 0) per_sm = occ;
     }
     if (p->warp_smem) {
-      const int by_smem = (int)(sm_bytes / (smem_bytes + 1024));
+      const int by_smem = (int)(sm_bytes / (smem_bytes + fixed + 1024));
       if (by_smem < per_sm) per_sm = by_smem;
     }
     if (mps_cap > 0 && mps_cap < per_sm) per_sm = mps_cap;
@@ -479,9 +552,10 @@ int deb_plan_create_ex(const deb_dims* dims, int max_modes, const deb_launch_cfg
     long nw = want < cap_warps ? want : cap_warps;
     p->warp_blocks = (int)nw;
     nslots = nw;
-    p->warp_smem_bytes = smem_bytes;
+    p->warp_smem_bytes = p->warp_smem ? smem_bytes : extra;
     // the attribute belongs to the kernel, not to the plan
-    if (p->warp_smem && ensure_warp_smem(dev, smem_bytes) != DEB_OK) {
+    if ((p->block_warps ? ensure_block_smem(dev, p->warp_smem_bytes)
+                        : (p->warp_smem ? ensure_warp_smem(dev, smem_bytes) : DEB_OK)) != DEB_OK) {
       delete p;
       return DEB_ERR_CUDA;
     }
@@ -650,11 +724,11 @@ int launch_forward(deb_plan* p, const double* d_tables, int ncosmo, int nset, in
     const int blocks = (int)(need < p->lane_blocks ? need : p->lane_blocks);
     forward_lane_kernel<<<blocks, kBlock, 0, s>>>(P);
   } else {
-    const int wpb = p->warp_block_warps;
-    long need = (items + wpb - 1) / wpb;
-    const int blocks = (int)(need < p->warp_blocks ? need : p->warp_blocks);
-    const size_t smem = p->warp_smem ? (size_t)p->warp_smem_bytes * wpb : 0;
-    forward_warp_kernel<<<blocks, 32 * wpb, smem, s>>>(P);
+    const int blocks = (int)(items < p->warp_blocks ? items : p->warp_blocks);
+    if (p->block_warps)
+      forward_block_kernel<kBlockWarps><<<blocks, 32 * kBlockWarps, (size_t)p->warp_smem_bytes, s>>>(P);
+    else
+      forward_warp_kernel<<<blocks, 32, p->warp_smem ? (size_t)p->warp_smem_bytes : 0, s>>>(P);
   }
   if (cudaGetLastError() != cudaSuccess) return DEB_ERR_CUDA;
   return DEB_OK;
