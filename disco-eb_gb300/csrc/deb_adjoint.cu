@@ -1,22 +1,21 @@
 // deb_adjoint.cu -- the discrete-adjoint kernel and its C ABI
 // (deb_plan_create_adjoint, deb_adjoint in include/discoeb_gb300.h).
 //
-// One warp per work item (cotangent seed, k-mode), pulled from a device
-// queue in order of recorded step counts, longest first.  A warp integrates
-// its mode backwards segment by segment: it recomputes the segment's states
-// from the checkpoint the recorded forward solve stored, then steps back
-// through them (deb_adjoint.cuh).  The forward slot, the adjoint vectors and
-// the segment states live in global memory (L2-resident for the warps in
-// flight); the bilinear forms, coefficient tables and scalar accumulators in
-// shared memory.  Replaces the reference's jax.jacfwd through diffrax
-// (perturbations.py:765) by one reverse sweep per mode.
+// One block of four warps per work item (cotangent seed, k-mode), pulled from
+// a device queue in order of recorded step counts, longest first
+// (deb_adjoint_block.cuh).  A block integrates its mode backwards segment by
+// segment: it recomputes the segment's states from the checkpoint the recorded
+// forward solve stored, then steps back through them.  As much of an item's
+// state as fits lives in shared memory, the rest in a global workspace
+// (L2-resident for the blocks in flight).  Replaces the reference's jax.jacfwd
+// through diffrax (perturbations.py:765) by one reverse sweep per mode.
 
 #include <cuda_runtime.h>
 
 #include <cstring>
 #include <mutex>
 
-#include "deb_adjoint.cuh"
+#include "deb_adjoint_block.cuh"
 #include "deb_internal.h"
 #include "discoeb_gb300.h"
 
@@ -51,39 +50,79 @@ struct AParams {
   int* queue;
   const int* order;          // modes, most recorded steps first
   deb::Dims D;
-  int shared_vectors;        // the NSHV hottest adjoint vectors in shared memory
+  int level;                 // what of an item's state lives in shared memory (adj_smem_doubles)
 };
 
-// Warps per SM the register allocation must leave room for: a build-time
-// option, 1 by default (255 registers).  Caps for 12 or 16 warps per SM were
-// measured slower at nvar 1098 (spills), and the plan runs fewer warps than
-// the registers allow anyway (the L2 fit).
-#ifndef DEB_ADJ_MIN_WARPS_PER_SM
-#define DEB_ADJ_MIN_WARPS_PER_SM 1
-#endif
+constexpr int kAdjWarps = 4, kAdjThreads = 32 * kAdjWarps;
+using AdjBlk = deb::AdjBlk<kAdjWarps>;
 
-__global__ void __launch_bounds__(32, DEB_ADJ_MIN_WARPS_PER_SM) adjoint_kernel(AParams P) {
+// per-block workspace in global memory, in doubles, after the slot, the
+// adjoint vectors and the segment states: theta differences and table sets
+constexpr long kThetaLen = (long)deb::NB * 9 * deb::MAXPAR;
+constexpr long kSetLen = (long)((2 * deb::MAXPAR * sizeof(deb::SetCtx) + 7) / 8);
+
+// doubles of dynamic shared memory: the scratch, the stages' momentum-bin
+// coefficients and, by level, 1: the slot without the stage vectors,
+// 2: and the stage vectors, 3: and the NSHV hottest adjoint vectors, 4: and
+// all adjoint vectors
+long adj_smem_doubles(const deb::Dims& D, int level) {
+  long d = deb::SC_LEN + (21L + 48L) * D.nq;
+  if (level >= 1) d += deb::hot_len(D);
+  if (level >= 2) d += deb::stage_len(D);
+  if (level == 3) d += (long)deb::NSHV * D.n;
+  if (level == 4) d += (long)deb::NAV * D.n;
+  return d;
+}
+
+// Two blocks per SM at 254 registers: eight warps of FP64 work hide each
+// other's latencies, and a register limit for more spills.  Measured against
+// one warp per item (one likelihood gradient from Python): nvar 323, 128 k, 8
+// outputs: 948 -> 247 ms; nvar 1098, 96 k, 64 outputs: 837 -> 227 ms.
+__global__ void __launch_bounds__(kAdjThreads, 2) adjoint_kernel(AParams P) {
   extern __shared__ double smem[];
-  const int lane = threadIdx.x & 31;
-  const deb::Grp<32> gp{lane};
-  const int n = P.D.n;
+  __shared__ __align__(16) unsigned char raw[sizeof(deb::AdjS)];   // no constructor runs
+  deb::AdjS& S = *reinterpret_cast<deb::AdjS*>(raw);
+  const int tid = threadIdx.x;
+  const int n = P.D.n, nq = P.D.nq;
+  double* const g = P.ws + (long)blockIdx.x * P.wslot;             // this block's global workspace
+  double* const g_av = g + deb::slot_len(P.D);
+  double* const g_seg = g_av + (long)deb::NAV * n;
+  double* const g_th = g_seg + (long)P.seg_cap * n;
+  double* sh = smem;
+  double* const sc = sh; sh += deb::SC_LEN;
+  double* const vqs = sh; sh += 21 * nq;
+  double* const vv = sh; sh += 48 * nq;
   deb::AWS<32> A;
-  A.w.p = P.ws + (long)blockIdx.x * P.wslot;
   A.w.n = n;
   A.w.misc0 = deb::V_K0 * n;
-  A.w.kp = A.w.p + deb::hot_len(P.D);
   A.w.dp = nullptr;
-  A.av = A.w.p + deb::slot_len(P.D);
-  A.seg = A.av + (long)deb::NAV * n;
+  A.w.p = P.level >= 1 ? sh : g;
+  if (P.level >= 1) sh += deb::hot_len(P.D);
+  A.w.kp = P.level >= 2 ? sh : g + deb::hot_len(P.D);
+  if (P.level >= 2) sh += deb::stage_len(P.D);
+  A.av = P.level == 4 ? sh : g_av;
+  A.shv = P.level == 3 ? sh : nullptr;
+  A.seg = g_seg;
   A.seg_cap = P.seg_cap;
-  A.sc = smem;
+  A.sc = sc;
   A.n = n;
-  A.shv = P.shared_vectors ? smem + deb::SC_LEN : nullptr;
+  deb::Blk<kAdjWarps> B{S.blk, A.w, vqs, P.D, c_rodas, tid, tid >> 5, tid & 31};
+  AdjBlk J{S, B, P.D, c_rodas, tid, tid >> 5, tid & 31};
+  J.lam = A.vec(deb::A_LAM).p; J.rb = A.vec(deb::A_RB).p; J.rbn = A.vec(deb::A_YOUT).p; J.ub = A.vec(deb::A_UB).p;
+  J.yh = A.vec(deb::A_YH).p; J.ye = A.vec(deb::A_YE).p; J.rho = A.vec(deb::A_RHO).p; J.u = A.vec(deb::A_TMP).p;
+  J.yo2 = A.vec(deb::A_YO2).p; J.kb = A.vec(deb::A_KB0).p;
+  J.vv = vv;
+  J.dth = g_th;
+  J.dth1 = g_th + (long)deb::NB * 8 * deb::MAXPAR;
+  J.sets = reinterpret_cast<deb::SetCtx*>(g_th + kThetaLen);
+  B.init_tables(c_tab);
+  J.init_lists();
   const long items = (long)P.nmode * P.nseed;
   for (;;) {
-    int q = 0;
-    if (lane == 0) q = atomicAdd(P.queue, 1);
-    q = __shfl_sync(0xffffffffu, q, 0);
+    if (tid == 0) S.blk.q = atomicAdd(P.queue, 1);
+    __syncthreads();
+    const int q = S.blk.q;
+    __syncthreads();
     if (q >= items) break;
     const int j = q / P.nseed, seed = q - j * P.nseed;
     const int m = P.order ? P.order[j] : j;
@@ -93,8 +132,8 @@ __global__ void __launch_bounds__(32, DEB_ADJ_MIN_WARPS_PER_SM) adjoint_kernel(A
     const int ci = P.cosmo ? P.cosmo[m] : 0;
     const double km = P.k[m];
     int st = deb::ST_BAD_INPUT;
+    deb::AdjItem it;
     if (ci >= 0 && ci < P.ncosmo && km > 0.0 && isfinite(km)) {
-      deb::AdjItem it;
       it.blob0 = P.tables + (long)ci * P.blob_len;
       it.blobs = P.tables_pm + (long)ci * 2 * P.npar * P.blob_len;
       it.blob_len = P.blob_len;
@@ -108,15 +147,14 @@ __global__ void __launch_bounds__(32, DEB_ADJ_MIN_WARPS_PER_SM) adjoint_kernel(A
       it.ck_stride = it.nrec >= 1 ? P.ckstride[m] : 1;
       it.gy = P.gy + item * P.nout * deb::NFIELD;
       it.k = km;
-      if (it.nrec >= 1 && it.nrec <= P.rec_len - 1)
-        st = deb::adjoint_item<32>(gp, it, P.D, c_tab, c_rodas, P.nout, A, gth);
+      if (it.nrec >= 1 && it.nrec <= P.rec_len - 1) st = J.run(it, P.nout, A, g_seg, P.seg_cap, gth);
     }
-    if (lane == 0) {
+    if (tid == 0) {
       P.status[item] = st;
       if (st != deb::ST_OK)
         for (int p = 0; p < P.npar; ++p) gth[p] = __longlong_as_double(0x7ff8000000000000LL);
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
@@ -167,19 +205,12 @@ int adj_upload_constants() {
   return DEB_OK;
 }
 
-constexpr size_t kAdjSmem = deb::SC_LEN * sizeof(double);
-// with the hottest adjoint vectors in shared memory as well
-size_t adj_smem_bytes(const deb::Dims& D, bool shared_vectors) {
-  return kAdjSmem + (shared_vectors ? (size_t)deb::NSHV * D.n * sizeof(double) : 0);
-}
-
 // the kernel's dynamic shared-memory limit, raised to at least bytes in the
 // current context (never lowered, so plans of other sizes keep working)
 std::mutex g_adj_smem_mu;
 unsigned long long g_adj_smem_ctx[64] = {0};
 size_t g_adj_smem_set[64] = {0};
 int adj_raise_smem(size_t bytes) {
-  if (bytes <= 48 * 1024) return DEB_OK;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DEB_ERR_CUDA;
   const unsigned long long ctx = deb_internal::current_ctx_id();
@@ -211,35 +242,28 @@ int deb_plan_create_adjoint(const deb_dims* dims, int max_items, int seg_cap, de
   if (dims->linear_solver != DEB_SOLVE_STRUCTURED || dims->return_full) return DEB_ERR_INVALID;
   int rc = adj_upload_constants();
   if (rc) return rc;
-  int dev = 0, nsm = 0, per_sm = 0;
+  int dev = 0, nsm = 0, optin = 0, sm_bytes = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return DEB_ERR_CUDA;
-  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return DEB_ERR_CUDA;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_kernel, 32, kAdjSmem) != cudaSuccess)
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
     return DEB_ERR_CUDA;
-  if (per_sm < 1) return DEB_ERR_INVALID;
-  {
-    // the vectors a warp touches every step: its forward slot, the adjoint
-    // vectors and one segment state
-    const deb::Dims D = deb::make_dims(dims->lmaxg, dims->lmaxgp, dims->lmaxr, dims->lmaxnu, dims->nqmax);
-    const long hot = (deb::slot_len(D) + (long)(deb::NAV + 1) * D.n) * (long)sizeof(double);
-    per_sm = deb_internal::l2_warps_per_sm(dev, nsm, hot, per_sm, 1.6);
-  }
-  // the hottest adjoint vectors in shared memory when that leaves the warps
-  // per SM chosen above (the kernel's attribute is only ever raised)
+  // Blocks per SM: two when there are items for them (the registers' limit),
+  // else one; the shared-memory level is the highest that leaves room for them.
   const deb::Dims Dm = deb::make_dims(dims->lmaxg, dims->lmaxgp, dims->lmaxr, dims->lmaxnu, dims->nqmax);
-  size_t smem = kAdjSmem;
-  {
-    int optin = 0, per_sm_bytes = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&per_sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-    const size_t want = adj_smem_bytes(Dm, true);
-    if (want <= (size_t)optin && (long)per_sm * (long)(want + 1024) <= (long)per_sm_bytes &&
-        adj_raise_smem(want) == DEB_OK)
-      smem = want;
+  const long fixed = (long)sizeof(deb::AdjS);
+  const int per_sm = max_items > nsm ? 2 : 1;
+  int level = 4;
+  for (; level > 0; --level) {
+    const long bytes = adj_smem_doubles(Dm, level) * (long)sizeof(double);
+    if (bytes + fixed <= optin && per_sm * (bytes + fixed + 1024) <= sm_bytes) break;
   }
+  const size_t smem = (size_t)adj_smem_doubles(Dm, level) * sizeof(double);
+  if (smem + fixed > (size_t)optin) return DEB_ERR_INVALID;
+  if (adj_raise_smem(smem) != DEB_OK) return DEB_ERR_CUDA;
   deb_plan* p = new deb_plan();
   p->adj_smem = (long)smem;
-  p->adj_shared = smem > kAdjSmem ? 1 : 0;
+  p->adj_level = level;
   p->D = deb::make_dims(dims->lmaxg, dims->lmaxgp, dims->lmaxr, dims->lmaxnu, dims->nqmax);
   p->nout = dims->nout;
   p->exec_mode = DEB_EXEC_WARP;
@@ -248,8 +272,9 @@ int deb_plan_create_adjoint(const deb_dims* dims, int max_items, int seg_cap, de
   p->slot_len = deb::slot_len(p->D);
   p->adj = 1;
   p->adj_seg_cap = seg_cap;
-  p->adj_wslot = p->slot_len + (long)(deb::NAV + seg_cap) * p->D.n;
-  // warps in flight: what the SMs hold, capped by the items and by 32 GiB
+  p->adj_wslot = p->slot_len + (long)(deb::NAV + seg_cap) * p->D.n + kThetaLen + kSetLen;
+  p->adj_wslot += p->adj_wslot & 1;
+  // blocks in flight: what the SMs hold, capped by the items and by 32 GiB
   long warps = (long)nsm * per_sm;
   const long mem_cap = (32L << 30) / (p->adj_wslot * 8);
   if (warps > mem_cap) warps = mem_cap;
@@ -288,13 +313,13 @@ int deb_adjoint(deb_plan* p, const double* d_tables, const double* d_tables_pm, 
   P.ckpt = d_ckpt; P.ck_cap = ck_cap; P.ckoff = d_ckoff; P.ckstride = d_ckstride; P.gy = d_gy; P.gth = d_gtheta; P.status = d_status;
   P.ws = p->adj_ws; P.wslot = p->adj_wslot; P.seg_cap = p->adj_seg_cap; P.queue = p->queue; P.order = p->order_dev;
   P.D = p->D;
-  P.shared_vectors = p->adj_smem > (long)kAdjSmem;
-  if (P.shared_vectors && adj_raise_smem((size_t)p->adj_smem) != DEB_OK) return DEB_ERR_CUDA;
+  P.level = p->adj_level;
+  if (adj_raise_smem((size_t)p->adj_smem) != DEB_OK) return DEB_ERR_CUDA;
   if (cudaMemsetAsync(p->queue, 0, sizeof(int), s) != cudaSuccess) return DEB_ERR_CUDA;
   rank_desc_adj_kernel<<<(nmode + 255) / 256, 256, 0, s>>>(d_nrec, nmode, p->order_dev);
   const long items = (long)nmode * nseed;
   const int blocks = (int)(items < p->adj_warps ? items : p->adj_warps);
-  adjoint_kernel<<<blocks, 32, (size_t)p->adj_smem, s>>>(P);
+  adjoint_kernel<<<blocks, kAdjThreads, (size_t)p->adj_smem, s>>>(P);
   return cudaGetLastError() == cudaSuccess ? DEB_OK : DEB_ERR_CUDA;
 }
 

@@ -223,7 +223,8 @@ struct Blk {
     __syncwarp();
   }
 
-  __device__ void produce(double t0, double dt, int vy, int vu) {
+  // all of it for one step; with_next: also the forward-mode background at y1
+  __device__ void produce(double t0, double dt, int vy, int vu, bool with_next) {
     const ModeConst& m = S.m;
     const Bg<Dual>& g0 = S.bg[S.cur];
     const double d = rcp(dt * R.gamma), idt = rcp(dt);
@@ -262,7 +263,7 @@ struct Blk {
     coefficients(kCoSplit + 1, 7, t0, dt);
     bar_arrive(BAR_CO2, NT);
     const double a1 = u + K(7, 0);
-    bg_dual(a1, S.bg[S.cur ^ 1]);
+    if (with_next) bg_dual(a1, S.bg[S.cur ^ 1]);
     // y1 of row 0, after the team has read the previous contents (it reads u[0] nowhere)
     if (lane == 0) V(vu, 0) = a1;
   }
@@ -938,40 +939,45 @@ struct Blk {
     team_sync();
   }
 
-  // One attempted step from (t0, y0 = vy) over dt: y1 into vu, stages and
-  // factors in the slot, S.ss the sum of squares of the scaled errors and
-  // S.bad whether y1 has a non-finite entry.  All threads of the block call
-  // it after a block barrier; it ends with one.
+  // The team's part of a step from (t0, y0 = vy): y1 into vu, stages and
+  // factors in the slot; whether this thread saw a non-finite entry of y1.
+  __device__ bool advance(double t0, double dt, int vy, int vu) {
+    const double idt = rcp(dt);
+    stage0(t0, dt, vy);
+    for (int s = 1; s < 8; ++s) stage(s, dt, idt, vy, vu);
+    // y1 = u + k8
+    const int n = D.n;
+    const double th = S.th, te = S.te;
+    bool bad = false;
+    for (int j = 2 + tid; j < n; j += TT) {
+      double kk = K(7, j);
+      kk += V(V_ZH, j) * th + V(V_ZE, j) * te;
+      K(7, j) = kk;
+      const double v = V(vu, j) + kk;
+      V(vu, j) = v;
+      bad = bad || !isfinite_(v);
+    }
+    team_sync();
+    if (wi == 2) {
+      row1(7);
+      if (lane == 0) {
+        const double v = V(vu, 1) + K(7, 1);
+        V(vu, 1) = v;
+        bad = bad || !isfinite_(v);
+      }
+    }
+    return bad;
+  }
+
+  // One attempted step from (t0, y0 = vy) over dt: S.ss the sum of squares of
+  // the scaled errors and S.bad whether y1 has a non-finite entry.  All
+  // threads of the block call it after a block barrier; it ends with one.
   __device__ void step(double t0, double dt, int vy, int vu, double rtol, double atol) {
     if (tid == 0) S.bad = 0;
     if (producer()) {
-      produce(t0, dt, vy, vu);
-    } else {
-      const double idt = rcp(dt);
-      stage0(t0, dt, vy);
-      for (int s = 1; s < 8; ++s) stage(s, dt, idt, vy, vu);
-      // y1 = u + k8
-      const int n = D.n;
-      const double th = S.th, te = S.te;
-      bool bad = false;
-      for (int j = 2 + tid; j < n; j += TT) {
-        double kk = K(7, j);
-        kk += V(V_ZH, j) * th + V(V_ZE, j) * te;
-        K(7, j) = kk;
-        const double v = V(vu, j) + kk;
-        V(vu, j) = v;
-        bad = bad || !isfinite_(v);
-      }
-      team_sync();
-      if (wi == 2) {
-        row1(7);
-        if (lane == 0) {
-          const double v = V(vu, 1) + K(7, 1);
-          V(vu, 1) = v;
-          bad = bad || !isfinite_(v);
-        }
-      }
-      if (bad) S.bad = 1;
+      produce(t0, dt, vy, vu, true);
+    } else if (advance(t0, dt, vy, vu)) {
+      S.bad = 1;
     }
     __syncthreads();
     if (wi == 0) {
