@@ -15,6 +15,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <cstdint>
@@ -263,29 +264,40 @@ constexpr int kBlockWarps = 4;
 inline long block_extra_bytes(const deb::Dims& D) { return 21L * D.nq * (long)sizeof(double); }
 inline long block_static_bytes() { return (long)sizeof(deb::BlkS); }
 
-// Groups of B consecutive modes sharing one step sequence (the reference's
-// batched variant): one warp per group, taken from the queue; the group's B
-// slots live in global memory and the warp steps its modes one after the
-// other inside each shared step (deb::group_solve).  A group whose modes are
-// not all valid or not all of one cosmology is marked BAD_INPUT.
-__global__ void __launch_bounds__(32) forward_group_kernel(KParams P, int B) {
-  const int lane = threadIdx.x & 31;
-  const long gwarp = blockIdx.x;
+// Groups of B <= 32 consecutive modes sharing one step sequence (the
+// reference's batched variant, deb::group_solve): a cluster per group, a warp
+// per mode, four warps to a block -- one for each sub-partition of an SM, whose
+// FP64 instructions take 64 cycles each whatever their lanes hold.  Inside a
+// shared step the warps work on their own; they meet once per attempt, when
+// every warp sums the group's error contributions (in mode order) out of the
+// blocks' shared memory and takes the same decision.  One warp walking the
+// group's modes took B times a mode's step: 672 ms for 256 modes of nvar 72 in
+// groups of 16, where this takes 46.  A group whose modes are not all valid or
+// not all of one cosmology is marked BAD_INPUT.
+constexpr int kGroupWarps = 4;
+
+__global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams P, int B) {
+  namespace cg = cooperative_groups;
+  extern __shared__ double smem[];
+  __shared__ double s_ss[2][kGroupWarps], s_t0[kGroupWarps];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int csize = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int b = rank * kGroupWarps + wi;           // this warp's mode of a group (none for b >= B)
   const deb::Grp<32> gp{lane};
   const int osz = P.ctl.return_full ? P.D.n : DEB_NOUT_FIELDS;
-  const int ngroup = P.nmode / B;
-  for (;;) {
-    int q = 0;
-    if (lane == 0) q = atomicAdd(P.queue, 1);
-    q = __shfl_sync(0xffffffffu, q, 0);
-    if (q >= ngroup) break;
-    const int m0 = q * B;
+  const int ngroup = P.nmode / B, nclust = (int)gridDim.x / csize, clust = (int)blockIdx.x / csize;
+  // value of mode j of the group in array p of its block
+  auto of_mode = [&](double* p, int j) -> double { return *cluster.map_shared_rank(p + j % kGroupWarps, j / kGroupWarps); };
+  for (int q = clust; q < ngroup; q += nclust) {
+    const int m0 = q * B, m = m0 + (b < B ? b : B - 1);
     const int ci = P.cosmo ? P.cosmo[m0] : 0;
     bool ok = ci >= 0 && ci < P.ncosmo;
-    for (int b = 0; b < B; ++b) {
-      const int m = m0 + b;
-      const double k = P.k[m];
-      ok = ok && (P.cosmo ? P.cosmo[m] : 0) == ci && k > 0.0 && isfinite(k);
+    for (int j = 0; j < B; ++j) {
+      const double kj = P.k[m0 + j];
+      ok = ok && (P.cosmo ? P.cosmo[m0 + j] : 0) == ci && kj > 0.0 && isfinite(kj);
+    }
+    if (b < B) {
       double* dst = P.y_out + (long)m * P.ctl.nout * osz;
       for (int i = lane; i < P.ctl.nout * osz; i += 32) dst[i] = __longlong_as_double(0x7ff8000000000000LL);
     }
@@ -293,29 +305,67 @@ __global__ void __launch_bounds__(32) forward_group_kernel(KParams P, int B) {
     if (ok) ok = deb::load_cosmo(P.tables + (long)ci * P.blob_len, P.blob_len, c0) && c0.nq == P.D.nq;
     deb::Run run;
     run.rec = nullptr; run.rec_cap = 0; run.nrec = 0; run.acc = 0; run.rej = 0; run.status = deb::ST_BAD_INPUT;
-    if (ok) {
+    if (ok) {                                      // the same for every warp of the cluster
       const double* tau_out = P.tau_out + (long)ci * P.ctl.nout;
-      auto ctx = [&](int b) {
+      auto ctx = [&](int j) {
         deb::ModeCtx<32> x;
         x.c = c0;
-        deb::mode_const(c0, P.k[m0 + b], x.m);
-        x.w.p = P.ws + (gwarp * B + b) * P.slot_len;
+        deb::mode_const(c0, P.k[m0 + j], x.m);
+        x.w.p = P.smem ? smem + (j % kGroupWarps) * P.slot_len
+                       : P.ws + ((long)clust * csize * kGroupWarps + j) * P.slot_len;
         x.w.n = P.D.n;
         x.w.misc0 = deb::V_K0 * P.D.n;
         x.w.kp = x.w.p + deb::hot_len(P.D);
         x.w.dp = nullptr;
         x.tau_out = tau_out;
-        x.yout = P.y_out + (long)(m0 + b) * P.ctl.nout * osz;
+        x.yout = P.y_out + (long)(m0 + j) * P.ctl.nout * osz;
         return x;
       };
-      deb::group_solve<32>(gp, P.D, c_tab, c_rodas, P.ctl, B, ctx, 1, run);
-    }
-    if (lane == 0)
-      for (int b = 0; b < B; ++b) {
-        const int m = m0 + b;
-        P.status[m] = run.status;
-        if (P.steps) { P.steps[2 * m] = run.acc; P.steps[2 * m + 1] = run.rej; }
+      const int step = csize * kGroupWarps;        // >= B: one pass of each loop below
+      for (int j = b; j < B; j += step) {
+        const deb::ModeCtx<32> x = ctx(j);
+        const double ts = deb::mode_start(x.c, x.m, P.ctl, x.tau_out);
+        if (lane == 0) s_t0[wi] = ts;
       }
+      cluster.sync();
+      double t0 = 1e300;
+      for (int j = 0; j < B; ++j) { const double ts = of_mode(s_t0, j); t0 = ts < t0 ? ts : t0; }
+      run.t0 = 0.0; run.T1 = 0.0; run.status = deb::ST_OK;
+      for (int j = b; j < B; j += step) {
+        const deb::ModeCtx<32> x = ctx(j);
+        deb::mode_begin<32>(gp, x.c, x.m, P.D, P.ctl, x.w, x.tau_out, run, t0);
+      }
+      // the modes' run.t0, T1 and steps are the group's, so all end together;
+      // a warp without a mode follows the first mode's flag (a negative entry)
+      for (int it = 0; it <= P.ctl.max_steps; ++it) {
+        bool go = run.t0 < run.T1;
+        if (go && run.steps >= P.ctl.max_steps) { run.status = deb::ST_MAX_STEPS; go = false; }
+        bool bad = false;
+        double ss = -1.0;
+        if (go)
+          for (int j = b; j < B; j += step) {
+            const deb::ModeCtx<32> x = ctx(j);
+            ss = deb::step_attempt<32>(gp, x.c, x.m, P.D, c_tab, c_rodas, P.ctl, x.w, run, bad);
+          }
+        if (b < B && lane == 0) s_ss[it & 1][wi] = ss;
+        cluster.sync();
+        if (of_mode(s_ss[it & 1], 0) < 0.0) break;
+        double sum = 0.0;
+        for (int j = 0; j < B; ++j) sum += of_mode(s_ss[it & 1], j);
+        const double err = sqrt(sum / (6.0 * B));
+        bool more = true;
+        for (int j = b; j < B; j += step) {
+          const deb::ModeCtx<32> x = ctx(j);
+          more = deb::step_decide<32>(gp, x.c, x.m, P.D, P.ctl, x.w, x.tau_out, x.yout, 1, run, err, bad);
+        }
+        if (!more) run.T1 = run.t0;
+      }
+      cluster.sync();                              // no block's values are read any more
+    }
+    if (b < B && lane == 0) {
+      P.status[m] = run.status;
+      if (P.steps) { P.steps[2 * m] = run.acc; P.steps[2 * m + 1] = run.rej; }
+    }
     __syncwarp();
   }
 }
@@ -378,6 +428,8 @@ unsigned long long g_consts_ctx[64] = {0};
 unsigned long long g_attr_ctx[64] = {0};
 // largest dynamic shared memory size set on forward_warp_kernel, per device
 long g_warp_smem_attr[64] = {0};
+unsigned long long g_group_attr_ctx[64] = {0};
+long g_group_smem_attr[64] = {0};
 unsigned long long g_block_attr_ctx[64] = {0};
 long g_block_smem_attr[64] = {0};
 
@@ -616,15 +668,30 @@ int deb_plan_create_grouped(const deb_dims* dims, int max_modes, int batch_size,
   p->slot_len = deb::slot_len(p->D);
   p->dense_len = 0;
   p->group_size = batch_size;
+  // a cluster of blocks of kGroupWarps warps per group; the slots in shared
+  // memory where a block's four fit, else in global memory
+  const int csize = (batch_size + kGroupWarps - 1) / kGroupWarps;
   const long groups = ((long)max_modes + batch_size - 1) / batch_size;
-  long warps = (long)nsm * kMaxWarpBlocksPerSM;
-  const long mem_cap = (16L << 30) / (p->slot_len * 8 * batch_size);
-  if (warps > mem_cap) warps = mem_cap;
-  if (warps > groups) warps = groups;
-  if (warps < 1) { delete p; return DEB_ERR_NOMEM; }
-  p->group_warps = (int)warps;
-  p->ws_bytes = (size_t)warps * batch_size * p->slot_len * sizeof(double);
-  if (cudaMalloc(&p->ws, p->ws_bytes) != cudaSuccess) { delete p; return DEB_ERR_NOMEM; }
+  const long block_bytes = kGroupWarps * p->slot_len * (long)sizeof(double);
+  int optin = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) { delete p; return DEB_ERR_CUDA; }
+  p->warp_smem = block_bytes + 1024 <= optin ? 1 : 0;
+  p->warp_smem_bytes = p->warp_smem ? block_bytes : 0;
+  if (ensure_smem(forward_group_kernel, g_group_attr_ctx, g_group_smem_attr, dev, p->warp_smem_bytes) != DEB_OK) {
+    delete p;
+    return DEB_ERR_CUDA;
+  }
+  // clusters in flight: two blocks per SM (registers), capped at 16 GiB of slots
+  long clusters = (long)nsm * 2 / csize;
+  if (!p->warp_smem) {
+    const long mem_cap = (16L << 30) / (block_bytes * csize);
+    if (clusters > mem_cap) clusters = mem_cap;
+  }
+  if (clusters > groups) clusters = groups;
+  if (clusters < 1) clusters = 1;
+  p->group_warps = (int)clusters;
+  p->ws_bytes = p->warp_smem ? 0 : (size_t)clusters * csize * block_bytes;
+  if (p->ws_bytes && cudaMalloc(&p->ws, p->ws_bytes) != cudaSuccess) { delete p; return DEB_ERR_NOMEM; }
   if (cudaMalloc(&p->queue, sizeof(int) * 4) != cudaSuccess) { cudaFree(p->ws); delete p; return DEB_ERR_NOMEM; }
   if (cudaMalloc(&p->order_dev, sizeof(int)) != cudaSuccess) {
     cudaFree(p->ws); cudaFree(p->queue); delete p; return DEB_ERR_NOMEM;
@@ -768,11 +835,22 @@ int deb_forward_grouped(deb_plan* p, const double* d_tables, int ncosmo, int blo
   P.ctl.max_steps = cfg->max_steps; P.ctl.hist_on_reject = cfg->hist_on_reject;
   P.ctl.dense = 0; P.ctl.return_full = 0; P.ctl.nout = p->nout;
   P.ctl.record = 0; P.ctl.replay = 0; P.ctl.step_ts = 0;
-  if (cudaMemsetAsync(p->queue, 0, sizeof(int), s) != cudaSuccess) return DEB_ERR_CUDA;
-  const int ngroup = nmode / p->group_size;
-  const int blocks = ngroup < p->group_warps ? ngroup : p->group_warps;
-  forward_group_kernel<<<blocks, 32, 0, s>>>(P, p->group_size);
-  if (cudaGetLastError() != cudaSuccess) return DEB_ERR_CUDA;
+  P.smem = p->warp_smem;
+  const int ngroup = nmode / p->group_size, csize = (p->group_size + kGroupWarps - 1) / kGroupWarps;
+  const int clusters = ngroup < p->group_warps ? ngroup : p->group_warps;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3((unsigned)(clusters * csize));
+  lc.blockDim = dim3(32 * kGroupWarps);
+  lc.dynamicSmemBytes = (size_t)p->warp_smem_bytes;
+  lc.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)csize;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  if (cudaLaunchKernelEx(&lc, forward_group_kernel, P, p->group_size) != cudaSuccess) return DEB_ERR_CUDA;
   return DEB_OK;
 }
 
