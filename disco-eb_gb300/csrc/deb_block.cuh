@@ -37,7 +37,7 @@ __device__ __forceinline__ void bar_sync(int id, int n) { __syncwarp(); asm vola
 __device__ __forceinline__ void bar_arrive(int id, int n) { __syncwarp(); asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 // coefficients of one stage's RHS that depend on (a, tau) only
-enum { CO_A = 0, CO_LA, CO_RHONU, CO_RHOQ, CO_IA, CO_IA2, CO_IAH, CO_AH, CO_RQ, CO_WQ, CO_CA2, CO_OP, CO_ITAU, CO_SG,
+enum { CO_A = 0, CO_LA, CO_RHONU, CO_RHOQ, CO_IA, CO_IA2, CO_IAH, CO_AH, CO_RQ, CO_WRQ, CO_CA2, CO_OP, CO_ITAU, CO_SG,
        NCO = CO_SG + NSIG };
 
 // Shared state of a block beside the mode's slot.
@@ -48,12 +48,14 @@ struct BlkS {
   Bg<Dual> bg[2];        // forward-mode background at the start of this step and of the next
   double co[8][NCO];
   double dv[NDV];        // h', eta', alpha, P1, 1 of the current stage
+  double dpnu;           // its momentum sum of the neutrino pressure
+  double cc[8][8];       // C_sq / dt
   double fun[6];         // functionals of Z_h, Z_e and of stage 0's solution
   double th, te;
   double ss;
   double dtt[3];         // d f / d tau of the truncation rows of photon T, P and massless nu
   Tab T;
-  double kap[NLEAD][NLT];
+  double kap[NLEAD][NLT], lk[NLEAD * NLT];   // lk: times the current stage's scalars
   short src[NLEAD][NLT], sig[NLEAD][NLT], tgt[NLEAD];
   int cur;               // which of bg[] is this step's
   int q, item, go, keep, more, nout_hit;
@@ -70,6 +72,7 @@ struct Blk {
   Dims D;
   const Rodas& R;
   int tid, wi, lane;
+  int ih, ie, ir1;   // this lane's elements of the h', eta' and row-1 lists (fewer than 33 entries)
 
   __device__ __forceinline__ bool producer() const { return wi == NW - 1; }
   __device__ __forceinline__ void team_sync() const { bar_sync(BAR_TEAM, TT); }
@@ -79,6 +82,10 @@ struct Blk {
 
   // once per launch: hierarchy coefficients and the lead rows' table in shared memory
   __device__ void init_tables(const Tab& T) {
+    const bool in = lane < D.nq + 6;
+    ih = in ? gather_index(D, GL_H, lane) : 0;
+    ie = in ? gather_index(D, GL_E, lane) : 0;
+    ir1 = in ? gather_index(D, GL_R1, lane) : 0;
     for (int l = tid; l < LMAX_TABLE + 2; l += NT) { S.T.lo[l] = T.lo[l]; S.T.up[l] = T.up[l]; }
     for (int e = tid; e < NLEAD * NLT; e += NT) {
       const int r = e / NLT, t = e - r * NLT;
@@ -201,7 +208,7 @@ struct Blk {
       const double rQ = m.gODE * g.rhoQ * g.a2;
       const double w1 = 1.0 + g.wQ;
       const double k = m.k, k2 = m.k2;
-      co[CO_IA] = g.ia; co[CO_IA2] = g.ia2; co[CO_IAH] = g.iaH; co[CO_AH] = g.aH; co[CO_RQ] = rQ; co[CO_WQ] = g.wQ;
+      co[CO_IA] = g.ia; co[CO_IA2] = g.ia2; co[CO_IAH] = g.iaH; co[CO_AH] = g.aH; co[CO_RQ] = rQ; co[CO_WRQ] = w1 * rQ;
       co[CO_CA2] = g.ca2; co[CO_OP] = g.opac; co[CO_ITAU] = itau;
       const double sg[NSIG] = {1.0, k, k2, g.opac, g.aH, g.a, g.aH * g.a, k2 * g.cs2, g.pb43 * g.opac,
                                -(D.lg + 1.0) * itau, -(D.lgp + 1.0) * itau, -(D.lr + 1.0) * itau, w1,
@@ -299,6 +306,10 @@ struct Blk {
       return dT;
     };
     for (int j = tid; j < n; j += TT) { V(V_ZH, j) = 0.0; V(V_ZE, j) = 0.0; }
+    if (wi == 2) {
+      const double idt = rcp(dt);
+      for (int e = lane; e < 64; e += 32) S.cc[e >> 3][e & 7] = R.C[e >> 3][e & 7] * idt;
+    }
     Dual drhonu = 0.0, dpnu = 0.0, fnu = 0.0;
     if (wi == 0) {
       for (int i = lane; i < nq; i += 32) {
@@ -424,9 +435,8 @@ struct Blk {
     sweep_many();
     team_sync();
     if (wi < 3) {
-      const int vec = wi == 0 ? V_ZH : (wi == 1 ? V_K0 : V_ZE);
       double sh, se;
-      functionals<32>(gp, D, w, vec, sh, se);
+      functionals_of(wi == 0 ? &V(V_ZH, 0) : (wi == 1 ? &K(0, 0) : &V(V_ZE, 0)), sh, se);
       if (lane == 0) { S.fun[2 * wi] = sh; S.fun[2 * wi + 1] = se; }
     }
     team_sync();
@@ -572,98 +582,56 @@ struct Blk {
     return r;
   }
 
-  // ------------------------------------------------------------------ M^-1 by parts (solve_M)
-  // neutrino chain ch of vector r (a full sweep and back-substitution)
-  __device__ __forceinline__ void chain_sweep(double* r, int ch) const {
-    const int nq = D.nq;
-    const double *UP = &V(V_UP, 0), *LO = &V(V_LO, 0), *PI = &V(V_PI, 0);
-    const int start = ch == 0 ? D.ir : D.iq0 + ch - 1;
-    const int stride = ch == 0 ? 1 : nq;
-    const int cnt = ch == 0 ? D.lr + 1 : D.lnu + 1;
-    int i = start + (cnt - 1) * stride;
-    double rn = r[i];
-    int j = cnt - 2;
-    for (; j >= 7; j -= 8) {
-      double rv[8], uv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { rv[q] = r[i - (q + 1) * stride]; uv[q] = UP[i - (q + 1) * stride]; }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { rn = rv[q] - uv[q] * rn; r[i - (q + 1) * stride] = rn; }
-      i -= 8 * stride;
+  // Elimination x_i = r_i - up_i x_prev downwards over cnt elements from i, a
+  // stride st apart; x is the element before them.  One dependent multiply-add
+  // per element (two upwards) with the next element's loads under it: 64 cycles
+  // each is the floor, 95 and 170 are measured.  Unrolling by four with padded
+  // trip counts was slower (5.9 against 4.9 thousand cycles for 18 elements down
+  // and up), a select on x inside the chain more so (107 against 64 per element).
+  static __device__ __forceinline__ void sweep_down(double* r, const double* up, int i, int st, int cnt, double x) {
+    double rv = r[i], uv = up[i];
+#pragma unroll 1
+    for (int j = 1; j <= cnt; ++j) {
+      const int nx = j < cnt ? i - st : i;
+      const double rn = r[nx], un = up[nx];
+      x = __fma_rn(-uv, x, rv);
+      r[i] = x;
+      i = nx; rv = rn; uv = un;
     }
-    for (; j >= 0; --j) {
-      i -= stride;
-      rn = r[i] - UP[i] * rn;
-      r[i] = rn;
-    }
-    double z = rn * PI[start];
-    r[start] = z;
-    int jb = 1;
-    for (; jb + 7 < cnt; jb += 8) {
-      double sv[8], lv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int ii = i + (q + 1) * stride;
-        sv[q] = r[ii] * PI[ii];
-        lv[q] = LO[ii];
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { z = sv[q] - lv[q] * z; r[i + (q + 1) * stride] = z; }
-      i += 8 * stride;
-    }
-    for (; jb < cnt; ++jb) {
-      i += stride;
-      z = r[i] * PI[i] - LO[i] * z;
+  }
+  // Back-substitution z_i = r_i / p_i - lo_i z_prev upwards from element i (the
+  // product lo_i z_prev is the rounded one)
+  static __device__ __forceinline__ void sweep_up(double* r, const double* pi, const double* lo, int i, int st, int cnt,
+                                                  double z) {
+    double rv = r[i], pv = pi[i], lv = lo[i];
+#pragma unroll 1
+    for (int j = 1; j <= cnt; ++j) {
+      const int nx = j < cnt ? i + st : i;
+      const double rn = r[nx], pn = pi[nx], ln = lo[nx];
+      z = __fma_rn(rv, pv, -__dmul_rn(lv, z));
       r[i] = z;
+      i = nx; rv = rn; pv = pn; lv = ln;
     }
+  }
+
+  // neutrino chain ch of vector r
+  __device__ __forceinline__ void chain_sweep(double* r, int ch) const {
+    const int st = ch == 0 ? 1 : D.nq, cnt = ch == 0 ? D.lr + 1 : D.lnu + 1;
+    const int first = ch == 0 ? D.ir : D.iq0 + ch - 1, top = first + (cnt - 1) * st;
+    sweep_down(r, &V(V_UP, 0), top - st, st, cnt - 1, r[top]);
+    const double z = r[first] * V(V_PI, first);
+    r[first] = z;
+    sweep_up(r, &V(V_PI, 0), &V(V_LO, 0), first + st, st, cnt - 1, z);
   }
 
   // photon tail t (0: T, 1: P) of vector r folded into its core row
   __device__ __forceinline__ void tail_fold(double* r, int t) const {
-    const double* UP = &V(V_UP, 0);
-    const int start = t == 0 ? 10 : D.igp + 3;
-    const int cnt = t == 0 ? D.lg - 2 : D.lgp - 2;
-    int i = start + (cnt - 1);
-    double rn = r[i];
-    int j = cnt - 2;
-    for (; j >= 7; j -= 8) {
-      double rv[8], uv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { rv[q] = r[i - (q + 1)]; uv[q] = UP[i - (q + 1)]; }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { rn = rv[q] - uv[q] * rn; r[i - (q + 1)] = rn; }
-      i -= 8;
-    }
-    for (; j >= 0; --j) {
-      i -= 1;
-      rn = r[i] - UP[i] * rn;
-      r[i] = rn;
-    }
-    r[start - 1] -= UP[start - 1] * rn;
+    const int start = t == 0 ? 10 : D.igp + 3, cnt = t == 0 ? D.lg - 2 : D.lgp - 2, top = start + cnt - 1;
+    sweep_down(r, &V(V_UP, 0), top - 1, 1, cnt, r[top]);   // the last element is the core row
   }
-
   __device__ __forceinline__ void tail_back(double* r, int t) const {
-    const double *LO = &V(V_LO, 0), *PI = &V(V_PI, 0);
-    const int start = t == 0 ? 10 : D.igp + 3;
-    const int cnt = t == 0 ? D.lg - 2 : D.lgp - 2;
-    double z = r[start - 1];
-    int j = 0;
-    for (; j + 7 < cnt; j += 8) {
-      double sv[8], lv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int i = start + j + q;
-        sv[q] = r[i] * PI[i];
-        lv[q] = LO[i];
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) { z = sv[q] - lv[q] * z; r[start + j + q] = z; }
-    }
-    for (; j < cnt; ++j) {
-      const int i = start + j;
-      z = r[i] * PI[i] - LO[i] * z;
-      r[i] = z;
-    }
+    const int start = t == 0 ? 10 : D.igp + 3, cnt = t == 0 ? D.lg - 2 : D.lgp - 2;
+    sweep_up(r, &V(V_PI, 0), &V(V_LO, 0), start, 1, cnt, r[start - 1]);
   }
 
   __device__ __forceinline__ int core_index(int j) const { return j < 5 ? 5 + j : D.igp + j - 5; }
@@ -705,13 +673,12 @@ struct Blk {
   // M^-1 of Z_h, Z_e and stage 0's vector
   __device__ void sweep_many() const {
     auto vec = [&](int v) -> double* { return v == 0 ? &V(V_ZH, 0) : (v == 1 ? &V(V_ZE, 0) : &K(0, 0)); };
-    const int nch = D.nq + 1;
     if (wi == 1) {
       photon_block(3, vec);
     } else {
       if (wi == 2 && lane < 3) scalar_blocks(vec(lane));
-      const int slot = wi == 0 ? lane : tid - 32;
-      for (int e = slot; e < 3 * nch; e += TT - 32) {
+      const int nch = D.nq + 1;
+      for (int e = wi == 0 ? lane : tid - 32; e < 3 * nch; e += TT - 32) {
         const int v = e / nch;
         chain_sweep(vec(v), e - v * nch);
       }
@@ -725,9 +692,67 @@ struct Blk {
       photon_block(1, [&](int) { return r; });
     } else {
       if (wi == 2 && lane == 0) scalar_blocks(r);
-      const int slot = wi == 0 ? lane : tid - 32;
-      for (int ch = slot; ch <= D.nq; ch += TT - 32) chain_sweep(r, ch);
+      for (int ch = wi == 0 ? lane : tid - 32; ch <= D.nq; ch += TT - 32) chain_sweep(r, ch);
     }
+  }
+
+  // sums of the momentum bins (one per lane, nq <= 32) in the order of
+  // Grp::sum3, without its additions of lanes that hold no bin
+  __device__ __forceinline__ void bin_sums(double& a, double& b, double& c) const {
+    const unsigned full = 0xffffffffu;
+    if (D.nq <= 8) {
+      const int g = lane >> 3, l = lane & 7;
+      const double vb = __shfl_sync(full, b, l), vc = __shfl_sync(full, c, l);
+      double v = g == 0 ? a : (g == 1 ? vb : vc);
+      if (D.nq > 4) v += __shfl_xor_sync(full, v, 4);
+      if (D.nq > 2) v += __shfl_xor_sync(full, v, 2);
+      v += __shfl_xor_sync(full, v, 1);
+      a = __shfl_sync(full, v, 0);
+      b = __shfl_sync(full, v, 8);
+      c = __shfl_sync(full, v, 16);
+    } else if (D.nq <= 16) {
+      const bool lo = lane < 16, q = (lane & 8) == 0;
+      const double vb = __shfl_xor_sync(full, b, 16);
+      const double k1 = lo ? a : vb, k2 = lo ? c : 0.0;
+      double k = (q ? k1 : k2) + __shfl_xor_sync(full, q ? k2 : k1, 8);
+      for (int o = 4; o > 0; o >>= 1) k += __shfl_xor_sync(full, k, o);
+      a = __shfl_sync(full, k, 0);
+      c = __shfl_sync(full, k, 8);
+      b = __shfl_sync(full, k, 16);
+    } else {
+      const Grp<32> gp{lane};
+      gp.sum3(a, b, c);
+    }
+  }
+
+  // g_h . r and g_e . r
+  __device__ __forceinline__ void functionals_of(const double* r, double& sh, double& se) const {
+    const int nq = D.nq;
+    const Grp<32> gp{lane};
+    double h = 0.0, e = 0.0;
+    if (nq + 6 <= 32) {
+      if (lane < nq + 6) {
+        h = w.m(gl_off(nq, GL_H) + lane) * r[ih];
+        e = w.m(gl_off(nq, GL_E) + lane) * r[ie];
+      }
+      if (nq + 6 <= 16) {
+        const unsigned full = 0xffffffffu;
+        const double eo = __shfl_xor_sync(full, e, 16);
+        double k = lane < 16 ? h : eo;
+        for (int o = 8; o > 0; o >>= 1) k += __shfl_xor_sync(full, k, o);
+        sh = __shfl_sync(full, k, 0);
+        se = __shfl_sync(full, k, 16);
+        return;
+      }
+    } else {
+      for (int t = lane; t < nq + 6; t += 32) {
+        h += w.m(gl_off(nq, GL_H) + t) * r[gather_index(D, GL_H, t)];
+        e += w.m(gl_off(nq, GL_E) + t) * r[gather_index(D, GL_E, t)];
+      }
+    }
+    gp.sum2(h, e);
+    sh = h;
+    se = e;
   }
 
   // ------------------------------------------------------------------ team: stages 1 .. 7
@@ -739,7 +764,7 @@ struct Blk {
     const double th = S.th, te = S.te;
     double a[SG], cc[SG];
 #pragma unroll
-    for (int q = 0; q < SG; ++q) { a[q] = R.a[SG][q]; cc[q] = R.C[SG][q] * idt; }
+    for (int q = 0; q < SG; ++q) { a[q] = R.a[SG][q]; cc[q] = S.cc[SG][q]; }
     for (int j = 2 + tid; j < n; j += TT) {
       double kq[SG];
 #pragma unroll
@@ -762,12 +787,31 @@ struct Blk {
     }
   }
 
+  // the RHS of row 1 at stage s, -(dgrho + 3 dgpres) a: read by nothing in this
+  // stage, so a warp without chains forms it during the solve
+  __device__ __forceinline__ void row1_rhs(int s, int vu) const {
+    if (lane == 0) {
+      const ModeConst& m = S.m;
+      const double* co = S.co[s];
+      const double dg = V(vu, 7), dr = V(vu, D.ir), dq = V(vu, D.n - 2), rptQ = co[CO_WRQ] * V(vu, D.n - 1);
+      const double dgpres = ((m.grhog * dg + m.grN * dr) * (1.0 / 3.0) + m.grM * (S.dpnu * (1.0 / 3.0))) * co[CO_IA2] +
+                            (m.cs2Q * co[CO_RQ] * dq + (m.cs2Q - co[CO_CA2]) * (3.0 * co[CO_AH] * rptQ * m.ik2));
+      const double f = -co[CO_A] * (S.dv[DV_P1] + 3.0 * dgpres);
+      K(s, 1) = __fma_rn(V(V_JC0, 1), K(s, 0), K(s, 1) + f);
+    }
+    __syncwarp();
+  }
+
   // row 1 of stage s's solution (never read by the RHS), by one warp
   __device__ __forceinline__ void row1(int s) const {
     const int nq = D.nq, o1 = gl_off(nq, GL_R1);
     const Grp<32> gp{lane};
     double s1 = 0.0;
-    for (int t = lane; t < nq + 6; t += 32) s1 += w.m(o1 + t) * K(s, gather_index(D, GL_R1, t));
+    if (nq + 6 <= 32) {
+      if (lane < nq + 6) s1 = w.m(o1 + lane) * K(s, ir1);
+    } else {
+      for (int t = lane; t < nq + 6; t += 32) s1 += w.m(o1 + t) * K(s, gather_index(D, GL_R1, t));
+    }
     s1 = gp.sum(s1);
     if (lane == 0) K(s, 1) = (K(s, 1) + s1) * w.m(M_SCAL + S_ID);
     __syncwarp();
@@ -827,25 +871,29 @@ struct Blk {
         dpnu = dpnu + wp0 * vq(s, 1)[i];
         fnu = fnu + wq * Y(iq1 + i);
       }
-      gp.sum3(drhonu, dpnu, fnu);
-      dpnu = dpnu * (1.0 / 3.0);
-      const double eta = Y(2), dc = Y(3), tc = Y(4), db = Y(5), tb = Y(6), dg = Y(7), tg = Y(8);
-      const double dr = Y(ir), tr = Y(ir + 1);
-      const double dq = Y(n - 2), tq = Y(n - 1);
-      const double rQ = co[CO_RQ], ia = co[CO_IA], ia2 = co[CO_IA2], iaH = co[CO_IAH];
-      double rptQ = (1.0 + co[CO_WQ]) * rQ * tq;
-      double dgrho = (m.gOc * dc + m.gOb * db) * ia + (m.grhog * dg + m.grN * dr + m.grM * drhonu) * ia2 + rQ * dq;
-      double hp = (2.0 * k2 * eta + dgrho) * iaH;
-      double dgtheta = (m.gOc * tc + m.gOb * tb) * ia + (m.g43g * tg + m.g43N * tr + m.grMk * fnu) * ia2 + rptQ;
-      double etap = 0.5 * dgtheta * m.ik2;
+      // dgrho (even lanes) and dgtheta (odd lanes) have one form
+      //   (Oc y1 + Ob y2) / a + (c3 y3 + c4 y4 + c5 S) / a^2 + c6 y6
+      const bool odd = (lane & 1) != 0;
+      const double y1 = Y(odd ? 4 : 3), y2 = Y(odd ? 6 : 5), y3 = Y(odd ? 8 : 7), y4 = Y(ir + (odd ? 1 : 0)),
+                   y6 = Y(n - (odd ? 1 : 2)), eta = Y(2);
+      const double c3 = odd ? m.g43g : m.grhog, c4 = odd ? m.g43N : m.grN, c5 = odd ? m.grMk : m.grM;
+      const double c6 = odd ? co[CO_WRQ] : co[CO_RQ], ia = co[CO_IA], ia2 = co[CO_IA2];
+      const double A = __fma_rn(m.gOc, y1, __dmul_rn(m.gOb, y2));
+      const double G = __fma_rn(c3, y3, __dmul_rn(c4, y4));
+      bin_sums(drhonu, dpnu, fnu);
+      const double T = __fma_rn(A, ia, __dmul_rn(__fma_rn(c5, odd ? fnu : drhonu, G), ia2));
+      const double d = odd ? __dadd_rn(T, __dmul_rn(c6, y6)) : __fma_rn(c6, y6, T);
+      // h' = (2 k^2 eta + dgrho) / aH; eta' = dgtheta / (2 k^2)
+      const double z = __dmul_rn(odd ? d : __fma_rn(2.0 * k2, eta, d), odd ? 0.5 * m.ik2 : co[CO_IAH]);
+      const double etap = __shfl_sync(0xffffffffu, z, 1);
       if (lane == 0) {
-        const double dgpres = ((m.grhog * dg + m.grN * dr) * (1.0 / 3.0) + m.grM * dpnu) * ia2 +
-                              (m.cs2Q * rQ * dq + (m.cs2Q - co[CO_CA2]) * (3.0 * co[CO_AH] * rptQ * m.ik2));
+        const double hp = z;
         S.dv[DV_HP] = hp;
         S.dv[DV_ETAP] = etap;
         S.dv[DV_ALPHA] = (hp + 6.0 * etap) * 0.5 * m.ik2;
-        S.dv[DV_P1] = dgrho + 3.0 * dgpres;
+        S.dv[DV_P1] = d;                           // dgrho (row1_rhs)
         S.dv[DV_ONE] = 1.0;
+        S.dpnu = dpnu;
       }
     } else {
       if (wi == 2) {
@@ -894,18 +942,20 @@ struct Blk {
         }
       }
     }
+    // the lead rows' coefficients, before the metric is known
+    if (wi == 2)
+      for (int e = lane; e < NLEAD * NLT; e += 32) S.lk[e] = (&S.kap[0][0])[e] * co[CO_SG + (&S.sig[0][0])[e]];
     team_sync();
-    if (wi == 0) {
-      if (lane < NLEAD && lane > 0) {
+    if (wi == 2) {
+      if (lane < NLEAD && lane > 1) {
         const int r = lane, tgt = S.tgt[r];
         double acc = 0.0;
 #pragma unroll
         for (int t = 0; t < NLT; ++t) {
           const int src = S.src[r][t];
-          const double x = src >= 0 ? Y(src) : S.dv[-1 - src];
-          acc = acc + (S.kap[r][t] * co[CO_SG + S.sig[r][t]]) * x;
+          acc = __fma_rn(S.lk[r * NLT + t], src >= 0 ? Y(src) : S.dv[-1 - src], acc);
         }
-        double t = K(s, tgt) + acc;
+        double t = __dadd_rn(K(s, tgt), acc);
         if (s <= 4) {
           if (r == 10) t = __fma_rn(dd, S.dtt[0], t);
           else if (r == 14) t = __fma_rn(dd, S.dtt[1], t);
@@ -913,27 +963,33 @@ struct Blk {
         }
         fin(tgt, t);
       }
-    } else if (wi == 1) {
+    } else if (wi == 0) {
       const double* kv = vq(s, 0);
-      const double hp = S.dv[DV_HP], etap = S.dv[DV_ETAP];
-      const double hp6 = hp * (1.0 / 6.0);
-      const double hp_eta = hp * (1.0 / 15.0) + 0.4 * etap;
+      const double hp6 = S.dv[DV_HP] * (1.0 / 6.0);
       for (int i = lane; i < nq; i += 32) {
         const double dlf = w.m(M_Q + Q_DLF * nq + i);
         double t = K(s, iq0 + i);
         t += -kv[i] * Y(iq1 + i) + hp6 * dlf;
         fin(iq0 + i, t);
-        t = K(s, iq2 + i);
+      }
+    } else if (wi == 1) {
+      const double* kv = vq(s, 0);
+      const double hp = S.dv[DV_HP], etap = S.dv[DV_ETAP];
+      const double hp_eta = hp * (1.0 / 15.0) + 0.4 * etap;
+      for (int i = lane; i < nq; i += 32) {
+        const double dlf = w.m(M_Q + Q_DLF * nq + i);
+        double t = K(s, iq2 + i);
         t += kv[i] * (2.0 * Y(iq1 + i) - 3.0 * Y(iq3 + i)) * 0.2 - hp_eta * dlf;
         fin(iq2 + i, t);
       }
     }
     team_sync();
     sweep_one(s);
+    if (wi == 2) row1_rhs(s, vu);
     team_sync();
     if (wi == 0) {
       double sh, se;
-      functionals<32>(gp, D, w, V_K0 + s, sh, se);
+      functionals_of(&K(s, 0), sh, se);
       woodbury(sh, se);
     }
     team_sync();
@@ -982,15 +1038,18 @@ struct Blk {
     __syncthreads();
     if (wi == 0) {
       const bool bad = S.bad != 0 || !isfinite_(V(vu, 0));
-      const int eidx[6] = {0, 2, 3, 5, 6, 7};
-      const double ew[6] = {1.0, S.m.k2, 1.0, 1.0, S.m.ik2, 1.0};
+      // the six entries of the error norm on six lanes, their squares summed in order
+      const int q = lane < 6 ? lane : 5;
+      const int j = q == 0 ? 0 : (q < 3 ? q + 1 : q + 2);
+      const double ew = q == 1 ? S.m.k2 : (q == 4 ? S.m.ik2 : 1.0);
+      const double y0 = fabs(V(vy, j));
+      const double y1 = bad ? y0 : fabs(V(vu, j));
+      const double sc = K(7, j) * rcp(__fma_rn(y0 > y1 ? y0 : y1, rtol, atol)) * ew;
       double ss = 0.0;
-      for (int q = 0; q < 6; ++q) {
-        const int j = eidx[q];
-        const double y0 = fabs(V(vy, j));
-        const double y1 = bad ? y0 : fabs(V(vu, j));
-        const double sc = K(7, j) * rcp(atol + (y0 > y1 ? y0 : y1) * rtol) * ew[q];
-        ss += sc * sc;
+#pragma unroll
+      for (int e = 0; e < 6; ++e) {
+        const double x = __shfl_sync(0xffffffffu, sc, e);
+        ss = __fma_rn(x, x, ss);
       }
       if (lane == 0) { S.ss = ss; S.bad = bad; }
       __syncwarp();
