@@ -4,17 +4,18 @@
 //
 // One block of one warp per parameter set (deb_tables_core.cuh holds the
 // per-set work).  The ionisation history is a sequential adaptive
-// integration over the sampling intervals and runs on lane 0; everything
-// indexed by a sample (neutrino momentum sums, HeII Saha fractions, sound
-// speeds, the Romberg integrals of d tau / d a, the spline coefficients) is
-// spread over the lanes.
+// integration over the sampling intervals; the lanes share the expressions of
+// each of its evaluations (deb_tables_warp.cuh).  Everything indexed by a
+// sample (neutrino momentum sums, HeII Saha fractions, sound speeds, the
+// Romberg integrals of d tau / d a, the spline coefficients) is spread over
+// the lanes.
 
 #include <cuda_runtime.h>
 
 #include <thread>
 #include <vector>
 
-#include "deb_tables_core.cuh"
+#include "deb_tables_warp.cuh"
 
 namespace {
 
@@ -22,7 +23,8 @@ using debt::TParams;
 
 __global__ void __launch_bounds__(32) tables_kernel(TParams P) {
   extern __shared__ double sh[];
-  debt::produce_set(P, blockIdx.x, threadIdx.x, 32, sh);
+  __shared__ double ion_sh[debt::IonWarp::SHARED];
+  debt::produce_set<debt::IonWarp>(P, blockIdx.x, threadIdx.x, 32, sh, ion_sh);
 }
 
 // tau(a) of each set at the output scale factors: the tau_of_a spline of

@@ -549,9 +549,24 @@ HD long tables_smem_doubles(int N, int NN) {
   return th + scr;
 }
 
+// The ionisation history's integrator: one lane (IonLane), or a warp whose
+// lanes all call it with the same arguments (IonWarp of deb_tables_warp.cuh).
+struct IonLane {
+  enum { SHARED = 0 };
+  const TC K;
+  const Bk& B;
+  HD IonLane(const TC& K_, const Bk& B_, double*, int) : K(K_), B(B_) {}
+  HD bool solve(double astart, double aend, const double* ystart, double rtol, double atol, int max_steps, double* out,
+                StepLog slog = StepLog(), const double* rep = nullptr, int nrep = 0, double rep_fin = 0.0) {
+    return solve_ionization(K, B, astart, aend, ystart, rtol, atol, max_steps, out, slog, rep, nrep, rep_fin);
+  }
+};
+
 // All tables of parameter set `set` into its blob; lanes lane, lane + G, ...
-// of a group of G share the sampled work; sh: tables_smem_doubles() doubles.
-HD void produce_set(const TParams& P, int set, int lane, int G, double* sh) {
+// of a group of G share the sampled work; sh: tables_smem_doubles() doubles;
+// ion_sh: Ion::SHARED doubles of the integrator.
+template <class Ion = IonLane>
+HD void produce_set(const TParams& P, int set, int lane, int G, double* sh, double* ion_sh = nullptr) {
   if (set >= P.nset) return;
   // the set's role with frozen step sequences: leaders in phase 1, the sets
   // that follow one in phase 2 (a leader index out of range or itself a
@@ -622,8 +637,10 @@ HD void produce_set(const TParams& P, int set, int lane, int G, double* sh) {
   const double Omegag = B.grhog / B.grhom;
   B.ODE = 1.0 - B.Ok - Omegar - Omegag - B.Om;
   const double taumin = P.amin / adotrad;
-  // ionisation history on lane 0 (thermodynamics_recfast.py:362-452)
-  if (lane == 0) {
+  // ionisation history (thermodynamics_recfast.py:362-452): every lane runs
+  // through it, lane 0 writes
+  {
+    Ion ion(K, B, ion_sh, lane);
     const double H = B.H0 / 100.0, HO = H * K[DEB_TC_BIG_H];
     const double mu_H = 1.0 / (1.0 - B.YHe);
     const double Nnow = 3.0 * HO * HO * B.Ob / (8.0 * K[DEB_TC_PI] * K[DEB_TC_G_N] * mu_H * K[DEB_TC_MH]);
@@ -642,18 +659,17 @@ HD void produce_set(const TParams& P, int set, int lane, int G, double* sh) {
       if (rep) {
         const int o0 = (int)rep[i], o1 = (int)rep[i + 1];
         if (o1 > o0 && o1 <= P.step_cap)
-          return solve_ionization(K, B, astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, StepLog(),
-                                  rep + 3 * N + 1 + 2 * o0, o1 - o0, rep[2 * N + 1 + i]) ? 0 : (int)DEB_BG_STEPS;
+          return ion.solve(astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, StepLog(), rep + 3 * N + 1 + 2 * o0,
+                           o1 - o0, rep[2 * N + 1 + i]) ? 0 : (int)DEB_BG_STEPS;
         if (o1 > P.step_cap) bad |= DEB_BG_UNRECORDED;
       }
       StepLog lg = slog;
       if (rec) lg.fin = rec + 2 * N + 1 + i;
-      return solve_ionization(K, B, astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, lg) ? 0
-                                                                                               : (int)DEB_BG_STEPS;
+      return ion.solve(astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, lg) ? 0 : (int)DEB_BG_STEPS;
     };
     for (int i = 0; i < N; ++i) {
       const double astart = P.a_th[i], aend = P.a_th[i + 1];
-      if (rec) rec[i] = pos;
+      if (rec && lane == 0) rec[i] = pos;
       const double zstart = 1.0 / astart - 1.0, zend = 1.0 / aend - 1.0;
       if (i == 0) {
         prev[0] = 1.0; prev[1] = 1.0; prev[2] = Tc * (1.0 + zstart); prev[3] = 0.0; prev[4] = 0.0;
@@ -665,7 +681,7 @@ HD void produce_set(const TParams& P, int set, int lane, int G, double* sh) {
       // the nominal values select
       int br = zend > 3500.0 ? 0 : (i > 0 && prev[1] > 0.99) ? 1 : (i > 0 && prev[0] > 0.99) ? 2 : 3;
       if (rep && br != 0) br = (int)rep[N + 1 + i];
-      if (rec) rec[N + 1 + i] = br;
+      if (rec && lane == 0) rec[N + 1 + i] = br;
       if (br == 0) {
         nw[0] = 1.0; nw[1] = 1.0; nw[2] = Tc * (1.0 + zend); nw[3] = 0.0; nw[4] = 0.0; nw[5] = -Tc * (1.0 + zend);
       } else if (br == 1) {
@@ -684,13 +700,16 @@ HD void produce_set(const TParams& P, int set, int lane, int G, double* sh) {
       } else {
         bad |= solve(i, astart, aend, nw);
       }
-      for (int j = 0; j < 6; ++j) { th[j * N + i] = nw[j]; prev[j] = nw[j]; }
+      for (int j = 0; j < 6; ++j) {
+        if (lane == 0) th[j * N + i] = nw[j];
+        prev[j] = nw[j];
+      }
     }
     if (rec) {
-      rec[N] = pos;
+      if (lane == 0) rec[N] = pos;
       if (pos > P.step_cap) bad |= DEB_BG_UNRECORDED;
     }
-    if (P.status) P.status[set] = bad | bad_leader;
+    if (P.status && lane == 0) P.status[set] = bad | bad_leader;
   }
   lane_sync(G);
   // per sample: x_e, c_s^2 a and the Romberg increment of tau
