@@ -562,24 +562,146 @@ struct IonLane {
   }
 };
 
+// parameters of a set, the densities of setup_background_evolution
+// (background.py:140-188) but the closure's; the neutrino mass / temperature
+HD double load_set(const TParams& P, const TC& K, int set, Bk& B) {
+  const double* pr = P.params + (long)set * DEB_BG_NPARAM;
+  B.Om = pr[DEB_BG_OMEGAM]; B.Ob = pr[DEB_BG_OMEGAB]; B.H0 = pr[DEB_BG_H0]; B.Tcmb = pr[DEB_BG_TCMB];
+  B.YHe = pr[DEB_BG_YHE]; B.Neff = pr[DEB_BG_NEFF]; B.Nmnu = pr[DEB_BG_NMNU]; B.w0 = pr[DEB_BG_W0];
+  B.wa = pr[DEB_BG_WA]; B.Ok = pr[DEB_BG_OMEGAK];
+  const double T2 = B.Tcmb * B.Tcmb, T4 = T2 * T2;
+  B.grhom = 3.33795017e-11 * B.H0 * B.H0;
+  B.grhog = 1.49594245e-13 * T4;
+  B.grhor = 3.39739477e-14 * T4;
+  B.fHe = B.YHe / (K[DEB_TC_MHE_MH] * (1.0 - B.YHe));
+  return pr[DEB_BG_MNU] * K[DEB_TC_C2OK] / B.Tcmb;
+}
+
+// neutrino density and (p non-null) pressure tables (background.py:47-68, 158-167)
+HD void nu_tables(const TParams& P, double amnu, double* rx, double* ry, double* px, double* py, int lane, int G) {
+  for (int i = lane; i < P.num_nu; i += G) {
+    const double a = P.a_nu[i];
+    double rho = 0.0, pn = 0.0;
+    for (int j = 0; j < P.nq_bg; ++j) {
+      const double q = P.qw_bg[j], w = P.qw_bg[P.nq_bg + j];
+      const double aq = a * amnu / q;
+      const double v = 1.0 / sqrt(1.0 + aq * aq);
+      rho += w / v;
+      pn += w * v / 3.0;
+    }
+    rx[i] = P.la_nu[i]; ry[i] = log(rho);
+    if (px) { px[i] = P.la_nu[i]; py[i] = log(pn); }
+  }
+}
+
+// closure (background.py:170-177), from the density spline of B
+HD void close_set(Bk& B) {
+  const double rhonu0 = exp(spl_ab(B.lx, B.ly, B.lS, B.nnu, 0.0));
+  const double Omegar = (B.Neff + B.Nmnu * rhonu0) * B.grhor / B.grhom;
+  const double Omegag = B.grhog / B.grhom;
+  B.ODE = 1.0 - B.Ok - Omegar - Omegag - B.Om;
+}
+
+// The ionisation history of a set (thermodynamics_recfast.py:362-452): every
+// lane runs through it, lane 0 writes.  rec: record to write (or null), rep:
+// record to follow (or null), th: [6][N] results (or null).  before(i) is
+// called ahead of interval i, after(i) behind it, when rec[0 .. i + 1] and the
+// steps of the interval are written.  Returns the DEB_BG_* bits.
+template <class Ion, class Before, class After>
+HD int history(const TParams& P, const TC& K, const Bk& B, double* ion_sh, double* rec, const double* rep, double* th,
+               int lane, Before before, After after) {
+  const int N = P.num_thermo;
+  Ion ion(K, B, ion_sh, lane);
+  const double H = B.H0 / 100.0, HO = H * K[DEB_TC_BIG_H];
+  const double mu_H = 1.0 / (1.0 - B.YHe);
+  const double Nnow = 3.0 * HO * HO * B.Ob / (8.0 * K[DEB_TC_PI] * K[DEB_TC_G_N] * mu_H * K[DEB_TC_MH]);
+  const double Tc = B.Tcmb;
+  int bad = 0;
+  double prev[6];
+  int pos = 0;
+  StepLog slog;
+  if (rec) { slog.steps = rec + 3 * N + 1; slog.pos = &pos; slog.cap = P.step_cap; }
+  // interval i: the leader's steps when it recorded all of them, adaptive
+  // otherwise (the leader did not integrate it, or its record overflowed)
+  auto solve = [&](int i, double astart, double aend, double* nw) {
+    if (rep) {
+      const int o0 = (int)rep[i], o1 = (int)rep[i + 1];
+      if (o1 > o0 && o1 <= P.step_cap)
+        return ion.solve(astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, StepLog(), rep + 3 * N + 1 + 2 * o0,
+                         o1 - o0, rep[2 * N + 1 + i]) ? 0 : (int)DEB_BG_STEPS;
+      if (o1 > P.step_cap) bad |= DEB_BG_UNRECORDED;
+    }
+    StepLog lg = slog;
+    if (rec) lg.fin = rec + 2 * N + 1 + i;
+    return ion.solve(astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, lg) ? 0 : (int)DEB_BG_STEPS;
+  };
+  if (rec && lane == 0) rec[0] = 0.0;
+  for (int i = 0; i < N; ++i) {
+    before(i);
+    const double astart = P.a_th[i], aend = P.a_th[i + 1];
+    const double zstart = 1.0 / astart - 1.0, zend = 1.0 / aend - 1.0;
+    if (i == 0) {
+      prev[0] = 1.0; prev[1] = 1.0; prev[2] = Tc * (1.0 + zstart); prev[3] = 0.0; prev[4] = 0.0;
+      prev[5] = -Tc * (1.0 + zstart);
+    }
+    double nw[6];
+    // the case of the thermal history (thermodynamics_recfast.py:362-452); a
+    // follower takes its leader's, as jax.jacfwd differentiates the branch
+    // the nominal values select
+    int br = zend > 3500.0 ? 0 : (i > 0 && prev[1] > 0.99) ? 1 : (i > 0 && prev[0] > 0.99) ? 2 : 3;
+    if (rep && br != 0) br = (int)rep[N + 1 + i];
+    if (rec && lane == 0) rec[N + 1 + i] = br;
+    if (br == 0) {
+      nw[0] = 1.0; nw[1] = 1.0; nw[2] = Tc * (1.0 + zend); nw[3] = 0.0; nw[4] = 0.0; nw[5] = -Tc * (1.0 + zend);
+    } else if (br == 1) {
+      const double rhs = exp(1.5 * log(K[DEB_TC_CR] * Tc / (1.0 + zend)) -
+                             K[DEB_TC_H_PLANCK] * K[DEB_TC_C] * K[DEB_TC_L_HE1_ION] / K[DEB_TC_KB] / (Tc * (1.0 + zend))) /
+                         Nnow * 4.0;
+      const double xHe0 = quad_root(rhs - 1.0, (1.0 + B.fHe) * rhs);
+      nw[0] = 1.0; nw[1] = (xHe0 - 1.0) / B.fHe; nw[2] = Tc * (1.0 + zend); nw[3] = 0.0; nw[4] = 0.0;
+      nw[5] = -Tc * (1.0 + zend);
+    } else if (br == 2) {
+      const double rhs = exp(1.5 * log(K[DEB_TC_CR] * Tc / (1.0 + zend)) - K[DEB_TC_CB1] / (Tc * (1.0 + zend))) / Nnow;
+      const double xH0 = quad_root(rhs, rhs);
+      bad |= solve(i, astart, aend, nw);
+      nw[0] = xH0;
+      nw[3] = 0.0;
+    } else {
+      bad |= solve(i, astart, aend, nw);
+    }
+    for (int j = 0; j < 6; ++j) {
+      if (th && lane == 0) th[j * N + i] = nw[j];
+      prev[j] = nw[j];
+    }
+    if (rec && lane == 0) rec[i + 1] = pos;
+    after(i);
+  }
+  if (rec && pos > P.step_cap) bad |= DEB_BG_UNRECORDED;
+  return bad;
+}
+
+// the leader of set `set` in a frozen production, -1: none (a leader index out
+// of range or itself a follower is refused with DEB_BG_BAD_LEADER and the set
+// runs adaptive)
+HD int leader_of(const TParams& P, int set, int& bad) {
+  bad = 0;
+  const int lead = P.leader ? P.leader[set] : -1;
+  if (lead >= 0 && (lead >= P.nset || P.leader[lead] >= 0)) {
+    bad = DEB_BG_BAD_LEADER;
+    return -1;
+  }
+  return lead;
+}
+
+struct NoHook { HD void operator()(int) const {} };
+
 // All tables of parameter set `set` into its blob; lanes lane, lane + G, ...
 // of a group of G share the sampled work; sh: tables_smem_doubles() doubles;
-// ion_sh: Ion::SHARED doubles of the integrator.
-template <class Ion = IonLane>
-HD void produce_set(const TParams& P, int set, int lane, int G, double* sh, double* ion_sh = nullptr) {
-  if (set >= P.nset) return;
-  // the set's role with frozen step sequences: leaders in phase 1, the sets
-  // that follow one in phase 2 (a leader index out of range or itself a
-  // follower is refused with DEB_BG_BAD_LEADER and the set runs adaptive)
-  int lead = -1, bad_leader = 0;
-  if (P.leader) {
-    lead = P.leader[set];
-    if ((lead >= 0) != (P.phase == 2)) return;
-    if (lead >= 0 && (lead >= P.nset || P.leader[lead] >= 0)) {
-      lead = -1;
-      bad_leader = DEB_BG_BAD_LEADER;
-    }
-  }
+// ion_sh: Ion::SHARED doubles of the integrator; rep: the record to follow (or
+// null), before(i) is called ahead of its interval i.
+template <class Ion, class Before>
+HD void produce_tables(const TParams& P, int set, int lane, int G, double* sh, double* ion_sh, double* rec,
+                       const double* rep, int bad_leader, Before before) {
   const int N = P.num_thermo, NN = P.num_nu;
   double* th = sh;                 // [6][N]: x_H, x_He, T_m, dx_H/da, dx_He/da, dT_m/da
   double* xe = sh + 6 * N;         // [N]
@@ -588,18 +710,8 @@ HD void produce_set(const TParams& P, int set, int lane, int G, double* sh, doub
   const TC K{P.consts};
   const double* pr = P.params + (long)set * DEB_BG_NPARAM;
   Bk B;
-  B.Om = pr[DEB_BG_OMEGAM]; B.Ob = pr[DEB_BG_OMEGAB]; B.H0 = pr[DEB_BG_H0]; B.Tcmb = pr[DEB_BG_TCMB];
-  B.YHe = pr[DEB_BG_YHE]; B.Neff = pr[DEB_BG_NEFF]; B.Nmnu = pr[DEB_BG_NMNU]; B.w0 = pr[DEB_BG_W0];
-  B.wa = pr[DEB_BG_WA]; B.Ok = pr[DEB_BG_OMEGAK];
-  const double mnu = pr[DEB_BG_MNU];
-  const double T2 = B.Tcmb * B.Tcmb, T4 = T2 * T2;
-  // setup_background_evolution (background.py:140-188)
-  B.grhom = 3.33795017e-11 * B.H0 * B.H0;
-  B.grhog = 1.49594245e-13 * T4;
-  B.grhor = 3.39739477e-14 * T4;
+  const double amnu = load_set(P, K, set, B);
   const double adotrad = sqrt((B.grhog + B.grhor * (B.Neff + B.Nmnu)) / 3.0);
-  const double amnu = mnu * K[DEB_TC_C2OK] / B.Tcmb;
-  B.fHe = B.YHe / (K[DEB_TC_MHE_MH] * (1.0 - B.YHe));
   double* blob = P.tables + (long)set * P.blob_len;
   // blob layout: header, 7 splines (x, y, S) in the order xe(loga),
   // cs2a(loga), lrhonu(loga), lpnu(loga), a(tau), tau(a), xe(tau), nodes,
@@ -613,104 +725,15 @@ HD void produce_set(const TParams& P, int set, int lane, int G, double* sh, doub
     sx[s] = blob + p; sy[s] = blob + p + sizes[s]; sS[s] = blob + p + 2 * sizes[s];
     p += 3L * sizes[s];
   }
-  // neutrino density and pressure tables (background.py:47-68, 158-167)
-  for (int i = lane; i < NN; i += G) {
-    const double a = P.a_nu[i];
-    double rho = 0.0, pn = 0.0;
-    for (int j = 0; j < P.nq_bg; ++j) {
-      const double q = P.qw_bg[j], w = P.qw_bg[P.nq_bg + j];
-      const double aq = a * amnu / q;
-      const double v = 1.0 / sqrt(1.0 + aq * aq);
-      rho += w / v;
-      pn += w * v / 3.0;
-    }
-    sx[2][i] = P.la_nu[i]; sy[2][i] = log(rho);
-    sx[3][i] = P.la_nu[i]; sy[3][i] = log(pn);
-  }
+  nu_tables(P, amnu, sx[2], sy[2], sx[3], sy[3], lane, G);
   lane_sync(G);
   for (int l = lane; l < 2; l += G) natural_S(sx[2 + l], sy[2 + l], sS[2 + l], NN, scr + l * 2 * NN, scr + l * 2 * NN + NN);
   lane_sync(G);
   B.lx = sx[2]; B.ly = sy[2]; B.lS = sS[2]; B.nnu = NN;
-  // closure (background.py:170-177)
-  const double rhonu0 = exp(spl_ab(sx[2], sy[2], sS[2], NN, 0.0));
-  const double Omegar = (B.Neff + B.Nmnu * rhonu0) * B.grhor / B.grhom;
-  const double Omegag = B.grhog / B.grhom;
-  B.ODE = 1.0 - B.Ok - Omegar - Omegag - B.Om;
+  close_set(B);
   const double taumin = P.amin / adotrad;
-  // ionisation history (thermodynamics_recfast.py:362-452): every lane runs
-  // through it, lane 0 writes
-  {
-    Ion ion(K, B, ion_sh, lane);
-    const double H = B.H0 / 100.0, HO = H * K[DEB_TC_BIG_H];
-    const double mu_H = 1.0 / (1.0 - B.YHe);
-    const double Nnow = 3.0 * HO * HO * B.Ob / (8.0 * K[DEB_TC_PI] * K[DEB_TC_G_N] * mu_H * K[DEB_TC_MH]);
-    const double Tc = B.Tcmb;
-    int bad = 0;
-    double prev[6];
-    // step record of this set (a leader) or of the set it follows
-    double* rec = (P.leader && P.steps && lead < 0 && !bad_leader) ? P.steps + (long)set * step_stride(P) : nullptr;
-    const double* rep = (P.leader && P.steps && lead >= 0) ? P.steps + (long)lead * step_stride(P) : nullptr;
-    int pos = 0;
-    StepLog slog;
-    if (rec) { slog.steps = rec + 3 * N + 1; slog.pos = &pos; slog.cap = P.step_cap; }
-    // interval i: the leader's steps when it recorded all of them, adaptive
-    // otherwise (the leader did not integrate it, or its record overflowed)
-    auto solve = [&](int i, double astart, double aend, double* nw) {
-      if (rep) {
-        const int o0 = (int)rep[i], o1 = (int)rep[i + 1];
-        if (o1 > o0 && o1 <= P.step_cap)
-          return ion.solve(astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, StepLog(), rep + 3 * N + 1 + 2 * o0,
-                           o1 - o0, rep[2 * N + 1 + i]) ? 0 : (int)DEB_BG_STEPS;
-        if (o1 > P.step_cap) bad |= DEB_BG_UNRECORDED;
-      }
-      StepLog lg = slog;
-      if (rec) lg.fin = rec + 2 * N + 1 + i;
-      return ion.solve(astart, aend, prev, P.rtol, P.atol, P.max_steps, nw, lg) ? 0 : (int)DEB_BG_STEPS;
-    };
-    for (int i = 0; i < N; ++i) {
-      const double astart = P.a_th[i], aend = P.a_th[i + 1];
-      if (rec && lane == 0) rec[i] = pos;
-      const double zstart = 1.0 / astart - 1.0, zend = 1.0 / aend - 1.0;
-      if (i == 0) {
-        prev[0] = 1.0; prev[1] = 1.0; prev[2] = Tc * (1.0 + zstart); prev[3] = 0.0; prev[4] = 0.0;
-        prev[5] = -Tc * (1.0 + zstart);
-      }
-      double nw[6];
-      // the case of the thermal history (thermodynamics_recfast.py:362-452); a
-      // follower takes its leader's, as jax.jacfwd differentiates the branch
-      // the nominal values select
-      int br = zend > 3500.0 ? 0 : (i > 0 && prev[1] > 0.99) ? 1 : (i > 0 && prev[0] > 0.99) ? 2 : 3;
-      if (rep && br != 0) br = (int)rep[N + 1 + i];
-      if (rec && lane == 0) rec[N + 1 + i] = br;
-      if (br == 0) {
-        nw[0] = 1.0; nw[1] = 1.0; nw[2] = Tc * (1.0 + zend); nw[3] = 0.0; nw[4] = 0.0; nw[5] = -Tc * (1.0 + zend);
-      } else if (br == 1) {
-        const double rhs = exp(1.5 * log(K[DEB_TC_CR] * Tc / (1.0 + zend)) -
-                               K[DEB_TC_H_PLANCK] * K[DEB_TC_C] * K[DEB_TC_L_HE1_ION] / K[DEB_TC_KB] / (Tc * (1.0 + zend))) /
-                           Nnow * 4.0;
-        const double xHe0 = quad_root(rhs - 1.0, (1.0 + B.fHe) * rhs);
-        nw[0] = 1.0; nw[1] = (xHe0 - 1.0) / B.fHe; nw[2] = Tc * (1.0 + zend); nw[3] = 0.0; nw[4] = 0.0;
-        nw[5] = -Tc * (1.0 + zend);
-      } else if (br == 2) {
-        const double rhs = exp(1.5 * log(K[DEB_TC_CR] * Tc / (1.0 + zend)) - K[DEB_TC_CB1] / (Tc * (1.0 + zend))) / Nnow;
-        const double xH0 = quad_root(rhs, rhs);
-        bad |= solve(i, astart, aend, nw);
-        nw[0] = xH0;
-        nw[3] = 0.0;
-      } else {
-        bad |= solve(i, astart, aend, nw);
-      }
-      for (int j = 0; j < 6; ++j) {
-        if (lane == 0) th[j * N + i] = nw[j];
-        prev[j] = nw[j];
-      }
-    }
-    if (rec) {
-      if (lane == 0) rec[N] = pos;
-      if (pos > P.step_cap) bad |= DEB_BG_UNRECORDED;
-    }
-    if (P.status && lane == 0) P.status[set] = bad | bad_leader;
-  }
+  const int bad = history<Ion>(P, K, B, ion_sh, rec, rep, th, lane, before, NoHook());
+  if (P.status && lane == 0) P.status[set] = bad | bad_leader;
   lane_sync(G);
   // per sample: x_e, c_s^2 a and the Romberg increment of tau
   // (thermodynamics_recfast.py:455-501)
@@ -766,6 +789,19 @@ HD void produce_set(const TParams& P, int set, int lane, int G, double* sh, doub
   lane_sync(G);
   // derived section: polynomial coefficients and FP32 knots of each spline
   for (int s = 0; s < 7; ++s) put_derived(blob, p, sx[s], sy[s], sS[s], sizes[s], lane, G);
+}
+
+// produce_tables of a set in its phase: with frozen step sequences the leaders
+// in phase 1, the sets that follow one in phase 2
+template <class Ion = IonLane>
+HD void produce_set(const TParams& P, int set, int lane, int G, double* sh, double* ion_sh = nullptr) {
+  if (set >= P.nset) return;
+  if (P.leader && (P.leader[set] >= 0) != (P.phase == 2)) return;
+  int bad = 0;
+  const int lead = leader_of(P, set, bad);
+  double* rec = (P.leader && P.steps && lead < 0 && !bad) ? P.steps + (long)set * step_stride(P) : nullptr;
+  const double* rep = (P.steps && lead >= 0) ? P.steps + (long)lead * step_stride(P) : nullptr;
+  produce_tables<Ion>(P, set, lane, G, sh, ion_sh, rec, rep, bad, NoHook());
 }
 
 }  // namespace debt

@@ -15,7 +15,8 @@
 // constants) and for the three derivative directions at once ((lane >> 2) % 3),
 // so the Jacobian costs twice a plain evaluation instead of four times.  What
 // depends on the scale factor alone is evaluated once per step, not once per
-// stage.  All branch conditions are on values every lane holds.
+// stage.  All branch conditions are on values every lane holds.  26 sets of 256
+// samples, leaders then followers: 252.6 ms on one lane, 79.6 ms.
 #pragma once
 
 #include "deb_tables_core.cuh"

@@ -12,7 +12,7 @@ its tables agree with theirs to rounding.
 ``[nset, blob_len]`` device tables out, optionally ``tau_of_a`` at given scale
 factors) and :func:`evolve_background_tables_host` (the same code on worker
 threads, numpy blobs out).  One RECFAST history is a long sequential chain of
-small FP64 steps: a CPU core builds a set in ~2 ms, one GPU lane in ~130 ms,
+small FP64 steps: a CPU core builds a set in ~2 ms, a GPU warp in ~40 ms,
 so the host producer is the faster one for the set counts of a gradient call.
 """
 from __future__ import annotations

@@ -403,7 +403,7 @@ int deb_evolve_background(const deb_bg_cfg* cfg, const double* d_params, int nse
 /* The same producer on the host cores (same code, compiled for the CPU): HOST
    buffers, nthreads worker threads over the sets (<= 0: one per hardware
    thread).  A RECFAST history is one long sequential chain of small FP64
-   steps, which a CPU core runs far faster than one GPU lane; for a few
+   steps, which a CPU core runs far faster than a GPU warp; for a few
    hundred sets this is the faster producer. */
 int deb_evolve_background_host(const deb_bg_cfg* cfg, const double* params, int nset, const double* consts,
                                const double* grid, double* tables, int blob_len, int* status, int nthreads);
@@ -424,11 +424,13 @@ int deb_evolve_background_host(const deb_bg_cfg* cfg, const double* params, int 
  *   d_steps  [nset, 3 num_thermo + 1 + 2 step_cap]     scratch: per leader
  *            the first step of each interval, the case of each interval, the
  *            branch word of its closing RHS evaluation, then an (end, branch
- *            word) pair per step, all as doubles; follower rows are unused.
+ *            word) pair per step, all as doubles; a follower's row is unused
+ *            or holds the same record again.
  *            step_cap = 16 num_thermo is ample at rtol 1e-3
  *            (DEB_BG_UNRECORDED reports an overflow).
  *
- * Two launches on `stream`: the leaders, then the followers.
+ * One launch on `stream` (each follower beside a repetition of its leader)
+ * for up to three sets per SM, else two: the leaders, then the followers.
  */
 int deb_evolve_background_frozen(const deb_bg_cfg* cfg, const double* d_params, int nset, const int* d_leader,
                                  const double* d_consts, const double* d_grid, double* d_steps, int step_cap,
