@@ -53,6 +53,7 @@ struct BlkS {
   double fun[6];         // functionals of Z_h, Z_e and of stage 0's solution
   double th, te;
   double ss;
+  double f0[6];          // entries -lo, up of the massless neutrinos' rows l = 0 .. 2
   double dtt[3];         // d f / d tau of the truncation rows of photon T, P and massless nu
   Tab T;
   double kap[NLEAD][NLT], lk[NLEAD * NLT];   // lk: times the current stage's scalars
@@ -307,6 +308,10 @@ struct Blk {
     };
     for (int j = tid; j < n; j += TT) { V(V_ZH, j) = 0.0; V(V_ZE, j) = 0.0; }
     if (wi == 2) {
+      if (lane == 0) {
+        S.f0[0] = 0.0; S.f0[1] = 0.25 * k2; S.f0[2] = 8.0 / 15.0;
+        S.f0[3] = 4.0 / 3.0; S.f0[4] = 0.5 * k2; S.f0[5] = 0.6 * k;
+      }
       const double idt = rcp(dt);
       for (int e = lane; e < 64; e += 32) S.cc[e >> 3][e & 7] = R.C[e >> 3][e & 7] * idt;
     }
@@ -368,32 +373,8 @@ struct Blk {
           w.m(M_SCAL + S_LEADD + NSIG + i) = dv[i].d;
         }
       }
-    } else if (wi == 1) {
-      // photon tails' factors, then the rows of the massive neutrinos without the metric
-      const double op = g.opac.v;
-      if (lane < 2) chain_factor<32>(m, D, S.T, w, d, itau, op, nq + 1 + lane);
-      for (int i = lane; i < nq; i += 32) {
-        const Dual kv = k * kvq(i);
-        const int jt = iq0 + lnu * nq + i;
-        put(iq1 + i, kv * (Y(iq0 + i) - 2.0 * Y(iq2 + i)) * (1.0 / 3.0));
-        const double dT = put_top(jt, kv * Y(jt - nq) - (lnu + 1.0) * itau * Y(jt), lnu);
-        w.m(M_Q + Q_DT * nq + i) = dT;
-      }
-    } else {
-      // neutrino chains' factors
-      for (int ch = tid - 64; ch <= nq; ch += HT - 32) chain_factor<32>(m, D, S.T, w, d, itau, g.opac.v, ch);
-    }
-    if (wi > 0) {
-      const int ngen = (lnu - 3) * nq;
-      for (int e = tid - 32; e < ngen; e += HT) {
-        const int l = 3 + e / nq, i = e - (l - 3) * nq;
-        const int j = iq3 + e;
-        put(j, k * kvq(i) * (S.T.lo[l] * Y(j - nq) - S.T.up[l] * Y(j + nq)));
-      }
-    }
-    team_sync();
-    auto scal = [&](int i) -> Dual { return Dual(w.m(M_SCAL + S_LEAD + i), w.m(M_SCAL + S_LEADD + i)); };
-    if (wi == 0) {
+      __syncwarp();
+      auto scal = [&](int i) -> Dual { return Dual(w.m(M_SCAL + S_LEAD + i), w.m(M_SCAL + S_LEADD + i)); };
       // lead rows
       if (lane < NLEAD) {
         const int r = lane, tgt = S.tgt[r];
@@ -410,27 +391,53 @@ struct Blk {
         else if (r > 0) put(tgt, acc);
         else V(V_JC0, 0) = acc.d;
       }
-    } else if (wi == 1) {
-      // massive-neutrino rows that read the metric
-      const Dual hp = scal(NSIG + DV_HP), etap = scal(NSIG + DV_ETAP);
-      const Dual hp6 = hp * (1.0 / 6.0);
-      const Dual hp_eta = hp * (1.0 / 15.0) + 0.4 * etap;
+      // massive-neutrino rows l = 0 .. 2 and lnu
+      const Dual hps = scal(NSIG + DV_HP), etaps = scal(NSIG + DV_ETAP);
+      const Dual hp6 = hps * (1.0 / 6.0);
+      const Dual hp_eta = hps * (1.0 / 15.0) + 0.4 * etaps;
       for (int i = lane; i < nq; i += 32) {
         const Dual kv = k * kvq(i);
         const double dlf = w.m(M_Q + Q_DLF * nq + i);
         put(iq0 + i, -kv * Y(iq1 + i) + hp6 * dlf);
         put(iq2 + i, kv * (2.0 * Y(iq1 + i) - 3.0 * Y(iq3 + i)) * 0.2 - hp_eta * dlf);
+        const int jt = iq0 + lnu * nq + i;
+        put(iq1 + i, kv * (Y(iq0 + i) - 2.0 * Y(iq2 + i)) * (1.0 / 3.0));
+        w.m(M_Q + Q_DT * nq + i) = put_top(jt, kv * Y(jt - nq) - (lnu + 1.0) * itau * Y(jt), lnu);
       }
-    } else if (wi == 2) {
-      // scalar blocks of W, functional coefficients, u_h and u_e
+    } else {
       Bg<double> gv;
       gv.a = g.a.v; gv.ia = g.ia.v; gv.ia2 = g.ia2.v; gv.a2 = g.a2.v; gv.la = g.la.v; gv.cs2 = g.cs2.v; gv.xe = g.xe.v;
       gv.rhonu = g.rhonu.v; gv.rhoQ = g.rhoQ.v; gv.aH = g.aH.v; gv.iaH = g.iaH.v; gv.wQ = g.wQ.v; gv.ca2 = g.ca2.v;
       gv.opac = g.opac.v; gv.pb43 = g.pb43.v;
-      factor_scalars(d, w00i, gv);
+      if (wi == 1) {
+        // photon tails' factors, the core's inverse, the momentum bins of the functionals
+        chain_entries_tails();
+        if (lane < 2) factor_chain(nq + 1 + lane, d, itau, gv.opac);
+        __syncwarp();
+        if (lane == 0) {
+          double core[64], de[4];
+          core_entries(m, S.T, gv, d, core, de);
+          core[36] -= w.m(M_SCAL + S_FT);
+          core[63] -= w.m(M_SCAL + S_FP);
+          for (int i = 0; i < 64; ++i) w.m(M_CORE + (i & 7) * 8 + (i >> 3)) = core[i];   // column-major
+        }
+        __syncwarp();
+        core_invert_warp();
+        factor_bins(gv);
+      } else {
+        // neutrino chains' factors; scalar blocks of W, functional coefficients
+        chain_entries_nu();
+        for (int ch = lane; ch <= nq; ch += 32) factor_chain(ch, d, itau, gv.opac);
+        factor_scalars(d, w00i, gv);
+      }
+      const int ngen = (lnu - 3) * nq;
+      for (int e = tid - 32; e < ngen; e += HT) {
+        const int l = 3 + e / nq, i = e - (l - 3) * nq;
+        const int j = iq3 + e;
+        put(j, k * kvq(i) * (S.T.lo[l] * Y(j - nq) - S.T.up[l] * Y(j + nq)));
+      }
     }
     team_sync();
-    if (wi == 1) core_invert_warp();
     // M^-1 of Z_h, Z_e and stage 0's vector together
     sweep_many();
     team_sync();
@@ -460,11 +467,72 @@ struct Blk {
     if (lane == 0) { S.th = th; S.te = te; }
   }
 
-  // the scalar blocks of W, the functionals' coefficients and row 1 (one
-  // lane), the momentum bins' coefficients and the columns u_h, u_e
+  // raw entries of the neutrino chains (by one warp) into V_LO, V_UP: what does
+  // not depend on the elimination is taken off its serial loop
+  __device__ __forceinline__ void chain_entries_nu() const {
+    const int nq = D.nq, nm = (D.lnu + 1) * nq, tot = nm + D.lr + 1;
+    const double k = S.m.k;
+    for (int e = lane; e < tot; e += 32) {
+      const bool mass = e < nm;
+      const int l = mass ? e / nq : e - nm, lmax = mass ? D.lnu : D.lr;
+      const bool fl = !mass && l <= 2;
+      const double kf = mass ? k * w.m(M_Q + Q_V * nq + e - l * nq) : (fl ? 1.0 : k);
+      const double el = l == lmax ? 1.0 : (fl ? S.f0[l] : S.T.lo[l]), eu = fl ? S.f0[3 + l] : S.T.up[l];
+      const int j = mass ? D.iq0 + e : D.ir + l;
+      V(V_LO, j) = -__dmul_rn(kf, el);
+      V(V_UP, j) = __dmul_rn(kf, eu);
+    }
+    __syncwarp();
+  }
+  // the same of the photon tails
+  __device__ __forceinline__ void chain_entries_tails() const {
+    const int nt = D.lg - 2, tot = nt + D.lgp - 2;
+    const double k = S.m.k;
+    for (int e = lane; e < tot; e += 32) {
+      const int l = 3 + (e < nt ? e : e - nt), j = (e < nt ? 7 : D.igp) + l;
+      V(V_LO, j) = -__dmul_rn(k, l == (e < nt ? D.lg : D.lgp) ? 1.0 : S.T.lo[l]);
+      V(V_UP, j) = __dmul_rn(k, S.T.up[l]);
+    }
+    __syncwarp();
+  }
+
+  // factors of chain ch from its raw entries (chain_factor of deb_core.cuh): a
+  // reciprocal and two dependent FP64 operations per element
+  __device__ __forceinline__ void factor_chain(int ch, double d, double itau, double op) const {
+    const Chain c = chain_of<32>(S.m, D, w, ch);
+    const double d_rest = c.attach >= 0 ? d + op : d;
+    double *UP = &V(V_UP, 0), *LO = &V(V_LO, 0), *PI = &V(V_PI, 0);
+    int i = c.start + (c.cnt - 1) * c.stride;
+    double lo = LO[i];
+    double pinv = rcp(__fma_rn(c.lmax + 1.0, itau, d_rest));
+    PI[i] = pinv;
+    LO[i] = __dmul_rn(lo, pinv);
+    i -= c.cnt > 1 ? c.stride : 0;
+    double up = UP[i], l2 = LO[i];
+#pragma unroll 1
+    for (int j = c.cnt - 2; j >= 0; --j) {
+      const int nx = j > 0 ? i - c.stride : i;
+      const double un = UP[nx], ln = LO[nx];
+      const double qf = __dmul_rn(up, pinv);
+      pinv = rcp(__fma_rn(-qf, lo, d_rest));
+      lo = l2;
+      UP[i] = qf;
+      PI[i] = pinv;
+      LO[i] = __dmul_rn(lo, pinv);
+      i = nx; up = un; l2 = ln;
+    }
+    if (c.attach >= 0) {
+      const double qa = 0.6 * S.m.k * pinv;
+      UP[c.attach] = qa;
+      w.m(M_SCAL + (ch == D.nq + 1 ? S_FT : S_FP)) = qa * lo;
+    }
+  }
+
+  // the scalar blocks of W, the functionals' coefficients, row 1 and the
+  // columns u_h, u_e but for the momentum bins (one lane)
   __device__ void factor_scalars(double d, double w00i, const Bg<double>& g) {
     const ModeConst& m = S.m;
-    const int n = D.n, nq = D.nq, iq0 = D.iq0, ir = D.ir;
+    const int n = D.n, nq = D.nq, ir = D.ir;
     const double a = g.a, iaH = g.iaH, h2 = 0.5 * m.ik2;
     if (lane == 0) {
       w.m(M_SCAL + S_D) = d;
@@ -491,9 +559,6 @@ struct Blk {
       w.m(o1 + 5) = -9.0 * (m.cs2Q - g.ca2) * g.aH * (1.0 + g.wQ) * rQ * a * m.ik2;
       double core[64], de[4];
       core_entries(m, S.T, g, d, core, de);
-      core[36] -= w.m(M_SCAL + S_FT);
-      core[63] -= w.m(M_SCAL + S_FP);
-      for (int i = 0; i < 64; ++i) w.m(M_CORE + (i & 7) * 8 + (i >> 3)) = core[i];   // column-major
       double a00 = de[0], a01 = de[1], a10 = de[2], a11 = de[3];
       double sw = 0.0;
       if (fabs(a10) > fabs(a00)) { double t0_ = a00, t1_ = a01; a00 = a10; a01 = a11; a10 = t0_; a11 = t1_; sw = 1.0; }
@@ -506,6 +571,12 @@ struct Blk {
       V(V_ZH, ir) = -2.0 / 3.0; V(V_ZH, ir + 2) = 4.0 / 15.0; V(V_ZH, n - 2) = -0.5 * (1.0 + g.wQ);
       V(V_ZE, 2) = 1.0; V(V_ZE, 9) = 1.6; V(V_ZE, ir + 2) = 1.6;
     }
+  }
+  // the momentum bins' coefficients and their rows of u_h and u_e (one warp)
+  __device__ void factor_bins(const Bg<double>& g) {
+    const ModeConst& m = S.m;
+    const int nq = D.nq, iq0 = D.iq0;
+    const double iaH = g.iaH, h2 = 0.5 * m.ik2;
     for (int i = lane; i < nq; i += 32) {
       const double v = w.m(M_Q + Q_V * nq + i);
       const double iv = rcp(v);
@@ -521,65 +592,56 @@ struct Blk {
   }
 
   // explicit inverse of the 8x8 core (core_invert of deb_core.cuh) with the
-  // 8 x 16 elimination spread over the warp: lane = row + 8 (column group),
-  // four columns a lane, so a step is one reciprocal, one multiply and four
-  // multiply-adds (a lane per row takes up to fifteen)
+  // 8 x 16 elimination spread over the warp: lane = row + 8 (column group), its
+  // four columns of (A | 1) in registers, so a step is one reciprocal, one
+  // multiply and four multiply-adds; the pivot row and column go through the
+  // slot.  Columns left of the pivot are eliminated too and read by nothing.
   __device__ void core_invert_warp() {
+    const unsigned full = 0xffffffffu;
     const int i = lane & 7, cg = lane >> 3;
-    auto A = [&](int r, int j) -> double& { return w.m(M_CORE + j * 8 + r); };
-    auto X = [&](int r, int j) -> double& { return w.m(M_CINV8 + j * 8 + r); };
-    for (int e = lane; e < 64; e += 32) X(e & 7, e >> 3) = ((e & 7) == (e >> 3)) ? 1.0 : 0.0;
+    double* A = &w.m(M_CORE);
+    double* X = &w.m(M_CINV8);
+    double* C = cg < 2 ? A + 32 * cg : X + 32 * (cg - 2);   // this group's columns
+    double e[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (cg >= 2) C[8 * c + i] = 4 * (cg - 2) + c == i ? 1.0 : 0.0;
+      e[c] = C[8 * c + i];
+    }
     __syncwarp();
     unsigned done = 0u;
-    int prow[8];
-    double pinv[8];
+    int prow = 0;
+    double pinv = 0.0;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
-      int key = (lane < 8 && !((done >> lane) & 1u)) ? abs_key(A(lane & 7, kk)) : -1;
-      int idx = lane;
-      for (int o = 4; o > 0; o >>= 1) {
-        const int ok = __shfl_xor_sync(0xffffffffu, key, o), oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        if (ok > key || (ok == key && oi < idx)) { key = ok; idx = oi; }
-      }
-      const int p = __shfl_sync(0xffffffffu, idx, 0);
+      // largest key, lowest row among equals
+      const int key = (lane < 8 && !((done >> lane) & 1u)) ? abs_key(A[kk * 8 + i]) : -1;
+      const int top = __reduce_max_sync(full, key);
+      const int p = __ffs(__ballot_sync(full, key == top)) - 1;
       done |= 1u << p;
-      prow[kk] = p;
-      const double pi = rcp(A(p, kk));
-      pinv[kk] = pi;
-      const double f = A(i, kk) * pi;
+      const double pv = A[kk * 8 + p], fv = A[kk * 8 + i];
+      double r[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) r[c] = C[8 * c + p];
       __syncwarp();
+      const double pi = rcp(pv), f = fv * pi;
       if (i != p) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const int j = 4 * cg + c;          // columns 0..7 of A, then of the inverse
-          if (j < 8) {
-            if (j > kk) A(i, j) = __fma_rn(-f, A(p, j), A(i, j));
-          } else {
-            X(i, j - 8) = __fma_rn(-f, X(p, j - 8), X(i, j - 8));
-          }
+          e[c] = __fma_rn(-f, r[c], e[c]);
+          C[8 * c + i] = e[c];
         }
       }
+      if (i == kk) { prow = p; pinv = pi; }
       __syncwarp();
     }
-    for (int e = lane; e < 64; e += 32) {
-      const int kk = e & 7, j = e >> 3;
-      A(kk, j) = X(prow_of(prow, kk), j) * pinv_of(pinv, kk);
-    }
-    __syncwarp();
-    for (int e = lane; e < 64; e += 32) X(e & 7, e >> 3) = A(e & 7, e >> 3);
-    __syncwarp();
-  }
-  static __device__ __forceinline__ int prow_of(const int* a, int k) {
-    int r = a[0];
+    double z[2];
 #pragma unroll
-    for (int q = 1; q < 8; ++q) r = k == q ? a[q] : r;
-    return r;
-  }
-  static __device__ __forceinline__ double pinv_of(const double* a, int k) {
-    double r = a[0];
+    for (int q = 0; q < 2; ++q) z[q] = X[8 * (cg + 4 * q) + prow] * pinv;
+    __syncwarp();
 #pragma unroll
-    for (int q = 1; q < 8; ++q) r = k == q ? a[q] : r;
-    return r;
+    for (int q = 0; q < 2; ++q) X[8 * (cg + 4 * q) + i] = z[q];
+    __syncwarp();
   }
 
   // Elimination x_i = r_i - up_i x_prev downwards over cnt elements from i, a
