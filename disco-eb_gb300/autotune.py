@@ -1,12 +1,13 @@
-"""Launch-shape autotuner for the warp-per-mode kernel.
+"""Launch-shape autotuner for the per-mode kernel.
 
 The kernel's speed depends on where a mode's eight Rodas5 stage vectors live
 and on how many modes share an SM (``deb_launch_cfg`` in
-``include/discoeb_gb300.h``): in shared memory a mode at nvar 323 takes 44 KB
-and five fit per SM; with the stage vectors in an L2-resident global array it
-takes 24 KB and up to eight fit (the register file's limit), at the price of
-an L2 round trip per stage access.  Which wins depends on the hierarchy sizes
-and on how much FP64 issue latency more resident warps hide, so it is
+``include/discoeb_gb300.h``): in shared memory a mode at nvar 323 takes 44 KB,
+with the stage vectors in an L2-resident global array 24 KB, at the price of
+an L2 round trip per stage access; registers allow four modes (blocks of four
+warps) per SM.  Fewer modes per SM run faster each, more use the FP64 unit
+better: which wins depends on the hierarchy sizes, the number of modes and how
+unequal they are, so it is
 measured, not guessed: :func:`tune` times one launch per candidate shape on
 the caller's own workload (CUDA events on the launching stream, after one
 untimed launch) and keeps the fastest.  Choices are remembered per (device

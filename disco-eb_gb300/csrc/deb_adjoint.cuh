@@ -1,8 +1,8 @@
 // deb_adjoint.cuh -- discrete adjoint (reverse mode) of the Rodas5 solve of
 // one k-mode on its recorded step sequence: d L / d theta for a cotangent of
 // the 20 output fields at every output time.  Host/device code like
-// deb_core.cuh: the CUDA kernel runs it with one warp per (seed, mode) item,
-// the test suite compiles it for the host.
+// deb_core.cuh: the CUDA kernel splits it over a block per (seed, mode) item
+// (deb_adjoint_block.cuh), the test suite compiles it for the host.
 //
 // What is differentiated.  The reference differentiates its solve with
 // jax.jacfwd (perturbations.py:765, DirectAdjoint; compute_matter_power in

@@ -21,7 +21,12 @@
 // others the hierarchies; in a solve the first takes the neutrino chains, the
 // second the photon tails and the photon-baryon core, the third the scalar
 // blocks.  The producer hands its coefficients over through two named barriers
-// (stages 1-3, stages 4-7).
+// (stages 1-3, stages 4-7).  In the first stage the factorisation runs beside
+// the right-hand side.
+//
+// Measured (whole calls, against one warp per mode): nvar 80, 64 modes 252 ->
+// 81 ms; nvar 323, 256 modes 423 -> 155 ms and 4096 modes 777 -> 583 ms; nvar
+// 265, 512 modes 201 -> 95 ms; nvar 72, 512 modes 54 -> 31 ms.
 #pragma once
 
 #include "deb_core.cuh"

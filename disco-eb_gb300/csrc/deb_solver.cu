@@ -1,14 +1,14 @@
 // deb_solver.cu -- CUDA kernels and the C ABI of include/discoeb_gb300.h.
 //
-// Execution model: one persistent grid sized to the device (blocks of 128
-// threads, a few blocks per SM); every thread owns one workspace slot and
-// pulls k-modes from a device-side queue (one atomicAdd per mode).  A mode is
-// integrated to completion by its thread, then the thread takes the next
-// queued mode, so modes with very different step counts (and modes of
-// different cosmologies) share the launch without lock-step waste.  Each
-// warp keeps its 32 slots interleaved in global memory (element e of lane l
-// at base + 32 e + l), so every vector access of the warp is one coalesced
-// 256-byte transaction.
+// Execution model: one persistent grid sized to the device; a block of four
+// warps (forward_block_kernel), a warp (forward_warp_kernel) or a thread
+// (forward_lane_kernel) owns one workspace slot and pulls k-modes from a
+// device-side queue.  A mode is integrated to completion, then the next queued
+// one is taken, so modes with very different step counts (and modes of
+// different cosmologies) share the launch without lock-step waste.  The lane
+// kernel's warps keep their 32 slots interleaved in global memory (element e of
+// lane l at base + 32 e + l), so every vector access is one coalesced 256-byte
+// transaction.
 //
 // Replaces jax.vmap(evolve_one_mode) of perturbations.py:980-987 (and the
 // lock-step while_loop it compiles to) for one GPU.

@@ -325,7 +325,7 @@ def evolve_perturbations_batched(*, param, aexp_out, kmin: float, kmax: float, n
     As in the reference, ``batch_size`` consecutive modes (of the geomspace
     grid) form a group that starts at the group's smallest start time and
     takes one shared step sequence, controlled by one error norm over all its
-    modes (``deb_forward_grouped``, one warp per group).  ``grouped=False``
+    modes (``deb_forward_grouped``, a warp per mode).  ``grouped=False``
     gives every mode its own start time and steps instead (the
     :func:`evolve_perturbations` semantics, the persistent per-mode kernel).
     ``batch_size`` must divide ``num_k`` as in the reference (1 to 32 here).

@@ -71,9 +71,10 @@ enum deb_linear_solver {
 
 /* how modes map onto the GPU */
 enum deb_exec_mode {
-  DEB_EXEC_AUTO = 0,        /* warp per mode for small batches, lane per mode for large ones */
+  DEB_EXEC_AUTO = 0,        /* block or warp per mode for small batches, lane per mode for large ones */
   DEB_EXEC_LANE = 1,        /* one thread per mode, state interleaved in global memory */
-  DEB_EXEC_WARP = 2         /* one warp per mode, state in shared memory */
+  DEB_EXEC_WARP = 2         /* a block of four warps (structured solver, nqmax <= 32) or one warp per mode,
+                               state in shared memory */
 };
 
 /* hierarchy sizes: the keyword arguments of evolve_perturbations (perturbations.py:926-930) */
@@ -114,13 +115,14 @@ int deb_plan_create(const deb_dims* dims, int max_modes, deb_plan** plan);
 int deb_plan_workspace_bytes(const deb_plan* plan, size_t* bytes);
 
 /*
- * Launch shape of the warp-per-mode kernel, no reference counterpart (the
+ * Launch shape of the per-mode kernel, no reference counterpart (the
  * reference's vmap has no launch shape).  A mode's state is 16 vectors of
  * nvar doubles plus a small block; the first 8 vectors and the block always
  * live in shared memory, the 8 Rodas5 stage vectors either there too
- * (DEB_STAGE_SHARED: 44 KB per mode at nvar 323, 5 modes per SM) or in an
+ * (DEB_STAGE_SHARED: 44 KB per mode at nvar 323) or in an
  * L2-resident global array (DEB_STAGE_GLOBAL: 24 KB of shared memory per
- * mode, up to 8 modes per SM, each stage access an L2 round trip).
+ * mode, each stage access an L2 round trip); registers allow 4 modes per SM
+ * (8 where one warp runs a mode).
  * modes_per_sm caps the modes in flight per SM (0: as many as fit).  Which
  * shape is faster depends on the hierarchy sizes; discoeb_gb300.autotune
  * times the candidates and picks one.  deb_plan_create uses
@@ -133,15 +135,16 @@ typedef struct deb_launch_cfg {
   int modes_per_sm;    /* cap on modes in flight per SM, 0 = no cap */
 } deb_launch_cfg;
 int deb_plan_create_ex(const deb_dims* dims, int max_modes, const deb_launch_cfg* launch, deb_plan** plan);
-/* The shape a plan resolved to, and its modes in flight (resident warps). */
+/* The shape a plan resolved to, and its modes in flight. */
 int deb_plan_launch_info(const deb_plan* plan, deb_launch_cfg* launch, int* modes_in_flight);
 
 /*
- * Scheduling hint, no reference counterpart.  The kernel hands modes to its
- * warps through a device-side queue; a launch ends when its last mode ends,
+ * Scheduling hint, no reference counterpart.  The kernel hands modes out
+ * through a device-side queue; a launch ends when its last mode ends,
  * and step counts differ by 60x across k, so handing out the most expensive
  * modes first shortens the tail.  d_order [nmode] (device) must be a
- * permutation of 0 .. nmode-1: queue position q takes mode d_order[q].
+ * permutation of 0 .. nmode-1: queue position q takes mode d_order[q].  The
+ * first block of each SM takes one of the first positions, one per SM.
  * Results do not depend on it.  The plan keeps the pointer (the array must
  * stay valid until every launch that reads it has finished) and applies it
  * to deb_forward / deb_forward_record launches with this nmode; NULL
