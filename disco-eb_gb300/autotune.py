@@ -21,10 +21,12 @@ import os
 
 from . import _native
 
-# (stage vectors, modes-per-SM cap); 0 = as many as fit.  "all_global" keeps
-# the whole mode state in L2-resident global memory: at nvar 1098 the shared
-# part alone (72 KB) limits the other shapes to three modes per SM.
-CANDIDATES = (("shared", 0), ("shared", 4), ("global", 0), ("global", 6), ("all_global", 0))
+# (stage vectors, modes-per-SM cap); 0 = as many as fit (four by registers).
+# One or two modes per SM win where a launch ends on its longest modes: 256 modes
+# of nvar 323 take 146 / 155 / 156 ms at 1 / 2 / 4, 4096 take 1051 / 685 / 578.
+# "all_global" keeps the whole mode state in L2-resident global memory: at nvar
+# 1098 the shared part alone is 72 KB.
+CANDIDATES = (("shared", 0), ("shared", 2), ("shared", 1), ("global", 0), ("all_global", 0))
 
 _chosen: dict = {}
 _loaded = False
