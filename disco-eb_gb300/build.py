@@ -13,7 +13,7 @@ ROOT = os.path.dirname(HERE)
 SRC = [os.path.join(HERE, "csrc", f) for f in ("deb_solver.cu", "deb_adjoint.cu", "deb_observables.cu", "deb_tables.cu")]
 HDRS = [os.path.join(HERE, "csrc", f) for f in ("deb_core.cuh", "deb_block.cuh", "deb_adjoint.cuh",
                                                  "deb_adjoint_block.cuh", "deb_tables_core.cuh", "deb_tables_warp.cuh",
-                                                 "deb_internal.h")]
+                                                 "deb_warp_sums.cuh", "deb_internal.h")]
 DEPS = SRC + HDRS + [os.path.join(ROOT, "include", "discoeb_gb300.h")]
 OUT = os.path.join(HERE, "_build", "libdiscoeb_gb300.so")
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"

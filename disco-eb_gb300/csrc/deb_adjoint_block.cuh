@@ -25,6 +25,7 @@
 
 #include "deb_adjoint.cuh"
 #include "deb_block.cuh"
+#include "deb_warp_sums.cuh"
 
 namespace deb {
 
@@ -193,34 +194,6 @@ struct AdjBlk {
   }
 
   // ------------------------------------------------------------------ producer
-  // Sums of N values over the warp, value i ending in the lanes with index
-  // bits i: the halves of the values are exchanged first, so N values take
-  // about N + 4 additions instead of 5 N.
-  template <int N>
-  static __device__ __forceinline__ void reduce_many(double* x, int lane, double* out) {
-    int cnt = N, own = 0, left = N;   // left: values of x in this lane that are not padding
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int half = (cnt + 1) >> 1;
-      const bool up = (lane & o) != 0;
-#pragma unroll
-      for (int i = 0; i < (N + 1) / 2; ++i) {
-        if (i < half) {
-          const double lo = x[i], hi = (i + half < cnt) ? x[i + half < N ? i + half : 0] : 0.0;
-          const double send = up ? lo : hi, keep = up ? hi : lo;
-          x[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-      }
-      if (cnt > 1) {
-        own += up ? half : 0;
-        left = up ? left - half : (left < half ? left : half);
-      }
-      cnt = half;
-    }
-    if (left > 0) out[own] = x[0];
-    __syncwarp();
-  }
-
   // coefficients of the stages at the nominal tables, Phi' and (at y0) Phi''
   __device__ void produce_nominal(double t0, double dt, double a0) {
     const ModeConst& m = S.blk.m;
@@ -497,7 +470,7 @@ struct AdjBlk {
       }
     }
     // slots 0 .. 4 of part[0] / part[1]
-    reduce_many<TWO ? 10 : 5>(p, lane, S.tmp[wi]);
+    warp_sums<TWO ? 10 : 5>(p, lane, S.tmp[wi]);
     if (lane < 5) {
       S.part[0][wi][lane] = S.tmp[wi][lane];
       if constexpr (TWO) S.part[1][wi][lane] = S.tmp[wi][5 + lane];
@@ -524,7 +497,7 @@ struct AdjBlk {
           q[17] -= xt * Y2[iq0 + lnu * nq + i];
         }
       }
-      reduce_many<TWO ? 18 : 10>(q, lane, S.tmp[3]);
+      warp_sums<TWO ? 18 : 10>(q, lane, S.tmp[3]);
       if (lane == 0) { S.hn = S.tmp[3][0]; S.en = S.tmp[3][1]; }
       if (lane < 8) {
         S.qs[0][lane] = S.tmp[3][2 + lane];
@@ -834,7 +807,7 @@ struct AdjBlk {
     }
     {
       double x[3] = {pc, pk, pf};
-      reduce_many<3>(x, lane, S.tmp[wi]);
+      warp_sums<3>(x, lane, S.tmp[wi]);
     }
     team_sync();
     const Coef<double>& E = *reinterpret_cast<const Coef<double>*>(S.C1);
@@ -899,7 +872,7 @@ struct AdjBlk {
       for (int p = 0; p < MAXPAR; ++p)
         if (p < npar) th[p] += t[p] * b;
     }
-    reduce_many<MAXPAR>(th, lane, S.tmp[wi]);
+    warp_sums<MAXPAR>(th, lane, S.tmp[wi]);
   }
 
   // a boundary's time adjoint into tau_start (scaled times), an output time or T1
