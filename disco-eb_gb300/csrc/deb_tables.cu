@@ -21,10 +21,13 @@ namespace {
 
 using debt::TParams;
 
+__host__ __device__ long set_smem_doubles(const TParams& P) {
+  return debt::set_smem_doubles<debt::IonWarp>(P.num_thermo, P.num_nu);
+}
+
 __global__ void __launch_bounds__(32) tables_kernel(TParams P) {
   extern __shared__ double sh[];
-  __shared__ double ion_sh[debt::IonWarp::SHARED];
-  debt::produce_set<debt::IonWarp>(P, blockIdx.x, threadIdx.x, 32, sh, ion_sh);
+  debt::produce_set<debt::IonWarp>(P, blockIdx.x, threadIdx.x, 32, sh);
 }
 
 // A frozen production in one launch: a block of two warps per set.  A set that
@@ -37,22 +40,21 @@ __global__ void __launch_bounds__(32) tables_kernel(TParams P) {
 // begins to be shared.  No block waits for another one.
 __global__ void __launch_bounds__(64) tables_pair_kernel(TParams P) {
   extern __shared__ double sh[];
-  __shared__ double ion_sh[2][debt::IonWarp::SHARED];
   const int set = blockIdx.x, wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int bad = 0;
   const int lead = debt::leader_of(P, set, bad);
   double* rec = P.steps + (long)set * debt::step_stride(P);
   if (lead < 0) {
-    if (wi == 0) debt::produce_tables<debt::IonWarp>(P, set, lane, 32, sh, ion_sh[0], bad ? nullptr : rec, nullptr, bad, debt::NoHook());
+    if (wi == 0) debt::produce_tables<debt::IonWarp>(P, set, lane, 32, sh, bad ? nullptr : rec, nullptr, bad, debt::NoHook());
     return;
   }
   // interval i is replayed while the leader's i + 1 is integrated
   auto meet = [](int) { __syncwarp(); asm volatile("bar.sync 1, 64;" ::: "memory"); };
   if (wi == 0) {
-    debt::produce_tables<debt::IonWarp>(P, set, lane, 32, sh, ion_sh[0], nullptr, rec, bad, meet);
+    debt::produce_tables<debt::IonWarp>(P, set, lane, 32, sh, nullptr, rec, bad, meet);
   } else {
     const int NN = P.num_nu;
-    double* x = sh + debt::tables_smem_doubles(P.num_thermo, NN);   // x, y, S, scratch [2]
+    double* x = sh + set_smem_doubles(P);   // x, y, S, scratch [2], the integrator's
     const debt::TC K{P.consts};
     debt::Bk B;
     const double amnu = debt::load_set(P, K, lead, B);
@@ -62,7 +64,7 @@ __global__ void __launch_bounds__(64) tables_pair_kernel(TParams P) {
     __syncwarp();
     B.lx = x; B.ly = x + NN; B.lS = x + 2 * NN; B.nnu = NN;
     debt::close_set(B);
-    debt::history<debt::IonWarp>(P, K, B, ion_sh[1], rec, nullptr, nullptr, lane, debt::NoHook(), meet);
+    debt::history<debt::IonWarp>(P, K, B, x + 5 * NN, rec, nullptr, nullptr, lane, debt::NoHook(), meet);
   }
 }
 
@@ -157,7 +159,7 @@ int deb_evolve_background(const deb_bg_cfg* cfg, const double* d_params, int nse
   const int rc = make_params(cfg, d_params, nset, d_consts, d_grid, d_tables, blob_len, d_status, P);
   if (rc) return rc;
   if (nset == 0) return DEB_OK;
-  const size_t smem = (size_t)debt::tables_smem_doubles(P.num_thermo, P.num_nu) * sizeof(double);
+  const size_t smem = (size_t)set_smem_doubles(P) * sizeof(double);
   if (smem > 48 * 1024) {
     if (cudaFuncSetAttribute(tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return DEB_ERR_INVALID;
@@ -185,7 +187,7 @@ int deb_evolve_background_frozen(const deb_bg_cfg* cfg, const double* d_params, 
   if (!d_leader || !d_steps || step_cap < 1) return DEB_ERR_INVALID;
   if (nset == 0) return DEB_OK;
   P.leader = d_leader; P.steps = d_steps; P.step_cap = step_cap;
-  const size_t smem = (size_t)debt::tables_smem_doubles(P.num_thermo, P.num_nu) * sizeof(double);
+  const size_t smem = (size_t)set_smem_doubles(P) * sizeof(double);
   if (smem > 48 * 1024) {
     if (cudaFuncSetAttribute(tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return DEB_ERR_INVALID;
@@ -196,8 +198,8 @@ int deb_evolve_background_frozen(const deb_bg_cfg* cfg, const double* d_params, 
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return DEB_ERR_CUDA;
-  const size_t pair = smem + 5 * (size_t)P.num_nu * sizeof(double), own = 2 * debt::IonWarp::SHARED * sizeof(double);
-  if (nset <= 3 * sms && pair + own <= (size_t)cap) {
+  const size_t pair = smem + (5 * (size_t)P.num_nu + debt::IonWarp::SHARED) * sizeof(double);
+  if (nset <= 3 * sms && pair <= (size_t)cap) {
     if (cudaFuncSetAttribute(tables_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair) != cudaSuccess)
       return DEB_ERR_INVALID;
     tables_pair_kernel<<<nset, 64, pair, (cudaStream_t)stream>>>(P);

@@ -695,18 +695,26 @@ HD int leader_of(const TParams& P, int set, int& bad) {
 
 struct NoHook { HD void operator()(int) const {} };
 
+// tables_smem_doubles with room for the integrator in the Thomas scratch, which
+// is free while the history runs: no shared memory of its own, so a set takes no
+// more of it than with one lane (num_thermo up to 1614 on 227 KB)
+template <class Ion>
+HD long set_smem_doubles(int N, int NN) {
+  const long d = tables_smem_doubles(N, NN), ion = 8L * N + Ion::SHARED;
+  return d > ion ? d : ion;
+}
+
 // All tables of parameter set `set` into its blob; lanes lane, lane + G, ...
-// of a group of G share the sampled work; sh: tables_smem_doubles() doubles;
-// ion_sh: Ion::SHARED doubles of the integrator; rep: the record to follow (or
-// null), before(i) is called ahead of its interval i.
+// of a group of G share the sampled work; sh: set_smem_doubles<Ion>() doubles;
+// rep: the record to follow (or null), before(i) is called ahead of its interval i.
 template <class Ion, class Before>
-HD void produce_tables(const TParams& P, int set, int lane, int G, double* sh, double* ion_sh, double* rec,
-                       const double* rep, int bad_leader, Before before) {
+HD void produce_tables(const TParams& P, int set, int lane, int G, double* sh, double* rec, const double* rep,
+                       int bad_leader, Before before) {
   const int N = P.num_thermo, NN = P.num_nu;
   double* th = sh;                 // [6][N]: x_H, x_He, T_m, dx_H/da, dx_He/da, dT_m/da
   double* xe = sh + 6 * N;         // [N]
   double* tau = xe + N;            // [N]
-  double* scr = tau + N;
+  double* scr = tau + N;           // Thomas scratch; the integrator's during the history
   const TC K{P.consts};
   const double* pr = P.params + (long)set * DEB_BG_NPARAM;
   Bk B;
@@ -732,7 +740,7 @@ HD void produce_tables(const TParams& P, int set, int lane, int G, double* sh, d
   B.lx = sx[2]; B.ly = sy[2]; B.lS = sS[2]; B.nnu = NN;
   close_set(B);
   const double taumin = P.amin / adotrad;
-  const int bad = history<Ion>(P, K, B, ion_sh, rec, rep, th, lane, before, NoHook());
+  const int bad = history<Ion>(P, K, B, scr, rec, rep, th, lane, before, NoHook());
   if (P.status && lane == 0) P.status[set] = bad | bad_leader;
   lane_sync(G);
   // per sample: x_e, c_s^2 a and the Romberg increment of tau
@@ -794,14 +802,14 @@ HD void produce_tables(const TParams& P, int set, int lane, int G, double* sh, d
 // produce_tables of a set in its phase: with frozen step sequences the leaders
 // in phase 1, the sets that follow one in phase 2
 template <class Ion = IonLane>
-HD void produce_set(const TParams& P, int set, int lane, int G, double* sh, double* ion_sh = nullptr) {
+HD void produce_set(const TParams& P, int set, int lane, int G, double* sh) {
   if (set >= P.nset) return;
   if (P.leader && (P.leader[set] >= 0) != (P.phase == 2)) return;
   int bad = 0;
   const int lead = leader_of(P, set, bad);
   double* rec = (P.leader && P.steps && lead < 0 && !bad) ? P.steps + (long)set * step_stride(P) : nullptr;
   const double* rep = (P.steps && lead >= 0) ? P.steps + (long)lead * step_stride(P) : nullptr;
-  produce_tables<Ion>(P, set, lane, G, sh, ion_sh, rec, rep, bad, NoHook());
+  produce_tables<Ion>(P, set, lane, G, sh, rec, rep, bad, NoHook());
 }
 
 }  // namespace debt
