@@ -205,24 +205,7 @@ int adj_upload_constants() {
   return DEB_OK;
 }
 
-// the kernel's dynamic shared-memory limit, raised to at least bytes in the
-// current context (never lowered, so plans of other sizes keep working)
-std::mutex g_adj_smem_mu;
-unsigned long long g_adj_smem_ctx[64] = {0};
-size_t g_adj_smem_set[64] = {0};
-int adj_raise_smem(size_t bytes) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DEB_ERR_CUDA;
-  const unsigned long long ctx = deb_internal::current_ctx_id();
-  std::lock_guard<std::mutex> lk(g_adj_smem_mu);
-  if (ctx != 0 && g_adj_smem_ctx[dev] == ctx && g_adj_smem_set[dev] >= bytes) return DEB_OK;
-  const size_t want = (g_adj_smem_ctx[dev] == ctx && g_adj_smem_set[dev] > bytes) ? g_adj_smem_set[dev] : bytes;
-  if (cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want) != cudaSuccess)
-    return DEB_ERR_CUDA;
-  g_adj_smem_ctx[dev] = ctx;
-  g_adj_smem_set[dev] = want;
-  return DEB_OK;
-}
+deb_internal::SmemLimit g_adj_smem;
 
 }  // namespace
 
@@ -260,7 +243,7 @@ int deb_plan_create_adjoint(const deb_dims* dims, int max_items, int seg_cap, de
   }
   const size_t smem = (size_t)adj_smem_doubles(Dm, level) * sizeof(double);
   if (smem + fixed > (size_t)optin) return DEB_ERR_INVALID;
-  if (adj_raise_smem(smem) != DEB_OK) return DEB_ERR_CUDA;
+  if (g_adj_smem.raise(adjoint_kernel, (long)smem) != cudaSuccess) return DEB_ERR_CUDA;
   deb_plan* p = new deb_plan();
   p->adj_smem = (long)smem;
   p->adj_level = level;
@@ -314,7 +297,7 @@ int deb_adjoint(deb_plan* p, const double* d_tables, const double* d_tables_pm, 
   P.ws = p->adj_ws; P.wslot = p->adj_wslot; P.seg_cap = p->adj_seg_cap; P.queue = p->queue; P.order = p->order_dev;
   P.D = p->D;
   P.level = p->adj_level;
-  if (adj_raise_smem((size_t)p->adj_smem) != DEB_OK) return DEB_ERR_CUDA;
+  if (g_adj_smem.raise(adjoint_kernel, p->adj_smem) != cudaSuccess) return DEB_ERR_CUDA;
   if (cudaMemsetAsync(p->queue, 0, sizeof(int), s) != cudaSuccess) return DEB_ERR_CUDA;
   rank_desc_adj_kernel<<<(nmode + 255) / 256, 256, 0, s>>>(d_nrec, nmode, p->order_dev);
   const long items = (long)nmode * nseed;

@@ -70,4 +70,29 @@ inline unsigned long long current_ctx_id() {
   return id + 1;   // 0 stays "unknown"
 }
 
+// The dynamic shared-memory limit of one kernel on each device.  The attribute
+// belongs to the kernel, so it is raised under a lock and never lowered: a
+// launch on another thread, or a plan made earlier, may need the larger value.
+// After a device reset (or with another context current) it is set again.
+struct SmemLimit {
+  std::mutex mu;
+  unsigned long long ctx[64] = {0};
+  long bytes[64] = {0};
+  template <class Kernel>
+  cudaError_t raise(Kernel* kernel, long want) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long id = current_ctx_id();
+    std::lock_guard<std::mutex> lock(mu);
+    const bool kept = dev >= 0 && dev < 64, same = kept && ctx[dev] == id;
+    if (same && id != 0 && bytes[dev] >= want) return cudaSuccess;
+    if (want < 48 * 1024) want = 48 * 1024;   // the limit that needs no attribute
+    if (same && want < bytes[dev]) want = bytes[dev];
+    const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+    if (rc == cudaSuccess && kept) { ctx[dev] = id; bytes[dev] = want; }
+    return rc;
+  }
+};
+
 }  // namespace deb_internal

@@ -444,19 +444,12 @@ __global__ void fp64_peak_kernel(double* out, int iters, double a, double b) {
   if (s == 12345.678) out[0] = s;  // keeps the chains live
 }
 
-// Per-device state that lives in a CUDA context (constant tables, kernel
-// attributes) is remembered together with the id of the context it was set
-// in: after cudaDeviceReset (or with another context current) the id
-// differs and the state is set again.  Guarded by g_state_mu.
+// Per-device state that lives in a CUDA context (the constant tables) is
+// remembered together with the id of the context it was set in: after
+// cudaDeviceReset (or with another context current) the id differs and the
+// state is set again.  Guarded by g_state_mu.
 std::mutex g_state_mu;
 unsigned long long g_consts_ctx[64] = {0};
-unsigned long long g_attr_ctx[64] = {0};
-// largest dynamic shared memory size set on forward_warp_kernel, per device
-long g_warp_smem_attr[64] = {0};
-unsigned long long g_group_attr_ctx[64] = {0};
-long g_group_smem_attr[64] = {0};
-unsigned long long g_block_attr_ctx[64] = {0};
-long g_block_smem_attr[64] = {0};
 
 int upload_constants() {
   int dev = 0;
@@ -480,27 +473,7 @@ int upload_constants() {
   return DEB_OK;
 }
 
-// Raise forward_warp_kernel's dynamic shared memory limit to at least
-// `bytes` in the current context (only ever raised, so that plans made
-// earlier with a larger slot stay launchable).
-template <class Kernel>
-int ensure_smem(Kernel* kernel, unsigned long long* attr_ctx, long* attr, int dev, long bytes) {
-  const unsigned long long ctx = deb_internal::current_ctx_id();
-  std::lock_guard<std::mutex> lock(g_state_mu);
-  const bool known = dev >= 0 && dev < 64 && ctx != 0 && attr_ctx[dev] == ctx;
-  if (known && attr[dev] >= bytes) return DEB_OK;
-  const long want = known && attr[dev] > bytes ? attr[dev] : bytes;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want) != cudaSuccess)
-    return DEB_ERR_CUDA;
-  if (dev >= 0 && dev < 64) { attr_ctx[dev] = ctx; attr[dev] = want; }
-  return DEB_OK;
-}
-int ensure_warp_smem(int dev, long bytes) {
-  return ensure_smem(forward_warp_kernel, g_attr_ctx, g_warp_smem_attr, dev, bytes);
-}
-int ensure_block_smem(int dev, long bytes) {
-  return ensure_smem(forward_block_kernel<kBlockWarps>, g_block_attr_ctx, g_block_smem_attr, dev, bytes);
-}
+deb_internal::SmemLimit g_warp_smem, g_group_smem, g_block_smem;
 
 }  // namespace
 
@@ -631,11 +604,10 @@ int deb_plan_create_ex(const deb_dims* dims, int max_modes, const deb_launch_cfg
     nslots = nw;
     p->warp_smem_bytes = p->warp_smem ? smem_bytes : extra;
     // the attribute belongs to the kernel, not to the plan
-    if ((p->block_warps ? ensure_block_smem(dev, p->warp_smem_bytes)
-                        : (p->warp_smem ? ensure_warp_smem(dev, smem_bytes) : DEB_OK)) != DEB_OK) {
-      delete p;
-      return DEB_ERR_CUDA;
-    }
+    cudaError_t e = cudaSuccess;
+    if (p->block_warps) e = g_block_smem.raise(forward_block_kernel<kBlockWarps>, p->warp_smem_bytes);
+    else if (p->warp_smem) e = g_warp_smem.raise(forward_warp_kernel, smem_bytes);
+    if (e != cudaSuccess) { delete p; return DEB_ERR_CUDA; }
   }
   const bool need_ws = mode == DEB_EXEC_LANE || !p->warp_smem;
   p->ws_bytes = (size_t)nslots * (need_ws ? p->slot_len : 0) * sizeof(double) + (size_t)nslots * p->dense_len * sizeof(double);
@@ -702,10 +674,7 @@ int deb_plan_create_grouped(const deb_dims* dims, int max_modes, int batch_size,
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) { delete p; return DEB_ERR_CUDA; }
   p->warp_smem = block_bytes + 1024 <= optin ? 1 : 0;
   p->warp_smem_bytes = p->warp_smem ? block_bytes : 0;
-  if (ensure_smem(forward_group_kernel, g_group_attr_ctx, g_group_smem_attr, dev, p->warp_smem_bytes) != DEB_OK) {
-    delete p;
-    return DEB_ERR_CUDA;
-  }
+  if (g_group_smem.raise(forward_group_kernel, p->warp_smem_bytes) != cudaSuccess) { delete p; return DEB_ERR_CUDA; }
   // clusters in flight: two blocks per SM (registers), capped at 16 GiB of slots
   long clusters = (long)nsm * 2 / csize;
   if (!p->warp_smem) {

@@ -15,6 +15,7 @@
 #include <thread>
 #include <vector>
 
+#include "deb_internal.h"
 #include "deb_tables_warp.cuh"
 
 namespace {
@@ -131,6 +132,8 @@ int make_params(const deb_bg_cfg* cfg, const double* params, int nset, const dou
   return DEB_OK;
 }
 
+deb_internal::SmemLimit g_tables_smem, g_pair_smem;
+
 // produce_set of every set on nthreads host threads (<= 0: one per hardware thread)
 void host_sets(const TParams& P, int nthreads) {
   const int nset = P.nset;
@@ -160,10 +163,7 @@ int deb_evolve_background(const deb_bg_cfg* cfg, const double* d_params, int nse
   if (rc) return rc;
   if (nset == 0) return DEB_OK;
   const size_t smem = (size_t)set_smem_doubles(P) * sizeof(double);
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return DEB_ERR_INVALID;
-  }
+  if (smem > 48 * 1024 && g_tables_smem.raise(tables_kernel, (long)smem) != cudaSuccess) return DEB_ERR_INVALID;
   tables_kernel<<<nset, 32, smem, (cudaStream_t)stream>>>(P);
   if (cudaGetLastError() != cudaSuccess) return DEB_ERR_CUDA;
   return DEB_OK;
@@ -188,10 +188,7 @@ int deb_evolve_background_frozen(const deb_bg_cfg* cfg, const double* d_params, 
   if (nset == 0) return DEB_OK;
   P.leader = d_leader; P.steps = d_steps; P.step_cap = step_cap;
   const size_t smem = (size_t)set_smem_doubles(P) * sizeof(double);
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      return DEB_ERR_INVALID;
-  }
+  if (smem > 48 * 1024 && g_tables_smem.raise(tables_kernel, (long)smem) != cudaSuccess) return DEB_ERR_INVALID;
   // one launch while all its blocks are resident, three per SM (tables_pair_kernel
   // has the times); a second wave would cost as much as the second launch
   int dev = 0, sms = 0, cap = 0;
@@ -200,8 +197,7 @@ int deb_evolve_background_frozen(const deb_bg_cfg* cfg, const double* d_params, 
     return DEB_ERR_CUDA;
   const size_t pair = smem + (5 * (size_t)P.num_nu + debt::IonWarp::SHARED) * sizeof(double);
   if (nset <= 3 * sms && pair <= (size_t)cap) {
-    if (cudaFuncSetAttribute(tables_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair) != cudaSuccess)
-      return DEB_ERR_INVALID;
+    if (pair > 48 * 1024 && g_pair_smem.raise(tables_pair_kernel, (long)pair) != cudaSuccess) return DEB_ERR_INVALID;
     tables_pair_kernel<<<nset, 64, pair, (cudaStream_t)stream>>>(P);
     return cudaGetLastError() == cudaSuccess ? DEB_OK : DEB_ERR_CUDA;
   }
