@@ -554,9 +554,14 @@ int deb_plan_create_ex(const deb_dims* dims, int max_modes, const deb_launch_cfg
     // a mode's whole slot in shared memory when 2 modes fit per SM, else only
     // the hot part (vectors before k1 + MISC) with k1..k8 in global memory
     // (L2-resident, lane-strided coalesced access)
-    // the structured solver runs a block of kBlockWarps warps per mode
-    // (up to 32 momentum bins: its sums over the bins take one lane per bin)
+    // the structured solver runs a block of kBlockWarps warps per mode (up to 32
+    // momentum bins, the counts its bits were compared for), but for a whole slot
+    // that was asked for in shared memory and fits it only without the block's
+    // own 8.7 KB and 21 nq doubles: one warp then, as with more bins
     p->block_warps = p->dense || p->D.nq > 32 ? 0 : kBlockWarps;
+    if (p->block_warps && stage_where == DEB_STAGE_SHARED &&
+        p->slot_len * 8 + block_extra_bytes(p->D) + block_static_bytes() > smem_optin)
+      p->block_warps = 0;
     const long extra = p->block_warps ? block_extra_bytes(p->D) : 0;       // dynamic, beside the slot
     const long fixed = p->block_warps ? block_static_bytes() : 0;
     smem_optin -= (int)fixed;
