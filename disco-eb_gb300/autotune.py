@@ -11,12 +11,15 @@ unequal they are, so it is
 measured, not guessed: :func:`tune` times one launch per candidate shape on
 the caller's own workload (CUDA events on the launching stream, after one
 untimed launch) and keeps the fastest.  Choices are remembered per (device
-name, hierarchy sizes, output count, solver) for the process and, when
-``DISCOEB_GB300_TUNE_CACHE`` names a JSON file, across processes.
+name, hierarchy sizes, output count, solver, number of modes within a factor
+of two) for the process and, when ``DISCOEB_GB300_TUNE_CACHE`` names a JSON
+file, across processes.  A launch of another number of modes does not take
+them: the best cap at 256 modes costs 1.8 times the best time at 4096 (below).
 """
 from __future__ import annotations
 
 import json
+import math
 import os
 
 from . import _native
@@ -31,13 +34,33 @@ CANDIDATES = (("shared", 0), ("shared", 2), ("shared", 1), ("global", 0), ("all_
 _chosen: dict = {}
 _loaded = False
 
+# Choices describe the kernel they were timed with: part of the key, so that a
+# file written for another kernel is not taken for this one's.
+KERNEL = "4 warps per mode"
+
 
 def _key(dims: _native.DebDims) -> str:
     import torch
 
     name = torch.cuda.get_device_name(torch.cuda.current_device())
-    return "|".join(str(v) for v in (name, dims.lmaxg, dims.lmaxgp, dims.lmaxr, dims.lmaxnu, dims.nqmax, dims.nout,
+    return "|".join(str(v) for v in (name, KERNEL, dims.lmaxg, dims.lmaxgp, dims.lmaxr, dims.lmaxnu, dims.nqmax, dims.nout,
                                      dims.return_full, dims.linear_solver))
+
+
+def _sms() -> int:
+    import torch
+
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+
+
+def mode_class(nmode: int, sms: int) -> int:
+    """Launches whose best shape is taken to be the same: up to one mode per
+    SM, then by powers of two of modes per SM."""
+    return max(0, math.ceil(math.log2(max(nmode, 1) / sms)))
+
+
+def _count_key(dims: _native.DebDims, nmode: int) -> str:
+    return f"{_key(dims)}|modes {mode_class(nmode, _sms())}"
 
 
 def _cache_path():
@@ -71,24 +94,37 @@ def _store():
         pass
 
 
-def chosen(dims: _native.DebDims):
-    """The tuned launch shape for these sizes, or None if not tuned yet."""
+def chosen(dims: _native.DebDims, nmode: int | None = None):
+    """The remembered launch shape for a launch of ``nmode`` modes of these
+    sizes, or None: the one tuned at that number of modes, else the one
+    remembered for any number.  Without ``nmode`` the latest choice for these
+    sizes, whatever its number of modes."""
     if dims.exec_mode == _native.EXEC_MODES["lane"]:
         return None
     _load()
-    return _chosen.get(_key(dims))
+    if not _chosen:
+        return None
+    key = _key(dims)
+    if nmode is not None:
+        return _chosen.get(_count_key(dims, nmode), _chosen.get(key))
+    found = [v for k, v in _chosen.items() if k == key or k.startswith(key + "|modes ")]
+    return found[-1] if found else None
 
 
-def remember(dims: _native.DebDims, launch) -> None:
+def remember(dims: _native.DebDims, launch, nmode: int | None = None) -> None:
+    """Keep a launch shape for launches of about ``nmode`` modes, or for any
+    number of modes that has no choice of its own."""
     _load()
-    _chosen[_key(dims)] = (str(launch[0]), int(launch[1]))
+    key = _key(dims) if nmode is None else _count_key(dims, nmode)
+    _chosen.pop(key, None)
+    _chosen[key] = (str(launch[0]), int(launch[1]))
     _store()
 
 
 def tune(dims: _native.DebDims, max_modes: int, launch_fn, candidates=CANDIDATES, stream=None):
-    """Time ``launch_fn(plan, stream)`` (one kernel launch on ``plan``) for
-    every candidate shape on a plan of ``max_modes`` modes; remember and
-    return ``(best_shape, {shape: ms})``.  Synchronises the device."""
+    """Time ``launch_fn(plan, stream)`` (the launches of one run on ``plan``)
+    for every candidate shape on a plan of ``max_modes`` modes; remember (for
+    that number of modes) and return ``(best_shape, {shape: ms})``.  Synchronises the device."""
     import torch
 
     s = stream if stream is not None else torch.cuda.current_stream()
@@ -113,5 +149,5 @@ def tune(dims: _native.DebDims, max_modes: int, launch_fn, candidates=CANDIDATES
     if not times:
         raise RuntimeError("autotune: no candidate launch shape could be planned")
     best = min(times, key=times.get)
-    remember(dims, best)
+    remember(dims, best, max_modes)
     return best, times

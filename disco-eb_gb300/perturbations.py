@@ -90,11 +90,11 @@ def get_plan(dims: _native.DebDims, nmode: int, launch=None) -> _native.Plan:
     """Cached plan for these hierarchy sizes with room for >= nmode modes.
 
     ``launch`` = (stage vectors, modes-per-SM cap) overrides the launch shape;
-    by default the shape :mod:`autotune` chose for these sizes is used, else
-    the library's default."""
+    by default the shape :mod:`autotune` chose for these sizes and about this
+    many modes is used, else the library's default."""
     torch = _torch()
     if launch is None:
-        launch = _autotune.chosen(dims)
+        launch = _autotune.chosen(dims, nmode)
     key = (torch.cuda.current_device(), dims.lmaxg, dims.lmaxgp, dims.lmaxr, dims.lmaxnu, dims.nqmax, dims.nout,
            dims.return_full, dims.linear_solver, dims.exec_mode, launch)
     p = _plans.get(key)
