@@ -283,7 +283,7 @@ class GradientProblem:
         self.d_dl = torch.empty((nm, no, len(self.theta)), dtype=torch.float64, device=dev)
         self.ode_names = [n for (n, _, _, _) in pert[0]]
         self.dims = _pt._dims(lmaxg, lmaxgp, lmaxr, lmaxnu, nqmax, no, False, linear_solver, "warp")
-        self.plan = _pt.get_plan(self.dims, (ns if self.method == "replay" else 1) * nm, launch)
+        self.plan = _pt.get_plan(self.dims, self._plan_modes(), launch)
         self.cfg = _pt._cfg(rtol, atol, pcoeff, icoeff, dcoeff, factormax, factormin, max_steps,
                             step_to_outputs=step_to_outputs)
         self.order = torch.as_tensor(_pt.schedule_order(self.host_k)).to(dev, torch.int32)
@@ -450,15 +450,35 @@ class GradientProblem:
                 g[:, j].index_add_(0, self.d_com_l, v)
         return g
 
+    def _replay(self, plan, s):
+        L = _native.load()
+        c = lambda t: ctypes.c_void_p(t.data_ptr())
+        _native.check(L.deb_replay(plan.ptr, c(self.d_tabs), self.nc, self.nset, self.blob_len, c(self.d_k), c(self.d_com),
+                                   self.nmode, c(self.d_taus), ctypes.byref(self.cfg), c(self.d_rec), self.rec_len,
+                                   c(self.d_nrec), c(self.d_ys), c(self.d_sts), ctypes.c_void_p(s.cuda_stream)),
+                      "deb_replay")
+
+    def _solves(self, plan, s):
+        """The launches of one run that take ``plan``: the record and, with
+        ``method="replay"``, the replay."""
+        self._record(plan, s)
+        if self.method == "replay":
+            self._replay(plan, s)
+
+    def _plan_modes(self):
+        return (self.nset if self.method == "replay" else 1) * self.nmode
+
     def tune(self, candidates=None):
-        """Choose the launch shape by timing the nominal recorded solve with
-        each candidate (:mod:`autotune`); the replay uses the same kernel.
-        Returns {shape: ms}."""
+        """Choose the launch shape by timing the solves of a run with each
+        candidate (:mod:`autotune`): the replay has ``nset`` times the
+        record's modes and its own best shape (128 modes of nvar 323: the
+        record takes 148 ms at any cap, both 553 / 397 / 379 ms at 1 / 2 / 4
+        modes per SM).  Returns {shape: ms}."""
         from . import autotune
 
-        best, times = autotune.tune(self.dims, self.nset * self.nmode, self._record,
-                                    candidates or autotune.CANDIDATES)
-        self.plan = _pt.get_plan(self.dims, self.nset * self.nmode, best)
+        n = self._plan_modes()
+        best, times = autotune.tune(self.dims, n, self._solves, candidates or autotune.CANDIDATES)
+        self.plan = _pt.get_plan(self.dims, n, best)
         self.graph = None
         return times
 
@@ -487,10 +507,7 @@ class GradientProblem:
             with torch.cuda.stream(s):
                 dl_ode = self.d_gth.permute(2, 1, 0)        # [npar, nmode, nout]
         else:
-            _native.check(L.deb_replay(self.plan.ptr, c(self.d_tabs), self.nc, self.nset, self.blob_len,
-                                       c(self.d_k), c(self.d_com), self.nmode, c(self.d_taus), ctypes.byref(self.cfg),
-                                       c(self.d_rec), self.rec_len, c(self.d_nrec), c(self.d_ys), c(self.d_sts), sp),
-                          "deb_replay")
+            self._replay(self.plan, s)
             if events:
                 events[2].record(s)
             with torch.cuda.stream(s):
