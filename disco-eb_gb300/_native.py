@@ -42,7 +42,7 @@ EXPORTS = ("deb_nvar", "deb_plan_create", "deb_plan_create_ex", "deb_plan_launch
            "deb_plan_set_order", "deb_forward", "deb_forward_static", "deb_tables_blob_len", "deb_evolve_background",
            "deb_evolve_background_host", "deb_evolve_background_frozen", "deb_evolve_background_frozen_host",
            "deb_tau_of_a", "deb_plan_create_grouped", "deb_forward_grouped",
-           "deb_forward_record", "deb_forward_record_ckpt", "deb_plan_create_adjoint", "deb_adjoint", "deb_replay",
+           "deb_forward_record", "deb_forward_record_ckpt", "deb_plan_create_adjoint", "deb_adjoint_launch_info", "deb_adjoint", "deb_replay",
            "deb_get_power", "deb_power_multipoles", "deb_density_velocity",
            "deb_power_kaiser", "deb_savgol_log", "deb_fftlog_phase",
            "deb_plan_destroy", "deb_measure_fp64_peak", "deb_error_string", "deb_version")
@@ -76,6 +76,7 @@ def load(path: str | None = None):
                                           ctypes.POINTER(DebSolverCfg), vp, vp, vp, vp, ctypes.c_int, vp, vp,
                                           ctypes.c_int, vp, vp, vp, vp]
     L.deb_plan_create_adjoint.argtypes = [ctypes.POINTER(DebDims), ctypes.c_int, ctypes.c_int, ctypes.POINTER(vp)]
+    L.deb_adjoint_launch_info.argtypes = [vp, ctypes.c_int, ctypes.POINTER(DebLaunchCfg), ctypes.POINTER(ctypes.c_int)]
     L.deb_adjoint.argtypes = [vp, vp, vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, vp, vp, vp, ctypes.c_int, vp, vp,
                               vp, ctypes.c_int, vp, vp, ctypes.c_int, vp, vp, vp, ctypes.c_int, vp, vp, vp]
     L.deb_replay.argtypes = [vp, vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, vp, vp, ctypes.c_int, vp,
@@ -137,10 +138,15 @@ class Plan:
             check(load().deb_plan_create_ex(ctypes.byref(dims), int(max_modes), ctypes.byref(lc), ctypes.byref(self.ptr)),
                   "deb_plan_create_ex")
 
-    def launch_info(self) -> dict:
-        """Resolved launch shape: stage vector placement, modes per SM, modes in flight."""
+    def launch_info(self, items: int | None = None) -> dict:
+        """Resolved launch shape: stage vector placement, modes per SM, modes in
+        flight; with ``items`` that of an adjoint launch of so many items."""
         lc, nf = DebLaunchCfg(), ctypes.c_int()
-        check(load().deb_plan_launch_info(self.ptr, ctypes.byref(lc), ctypes.byref(nf)), "deb_plan_launch_info")
+        if items is None:
+            check(load().deb_plan_launch_info(self.ptr, ctypes.byref(lc), ctypes.byref(nf)), "deb_plan_launch_info")
+        else:
+            check(load().deb_adjoint_launch_info(self.ptr, int(items), ctypes.byref(lc), ctypes.byref(nf)),
+                  "deb_adjoint_launch_info")
         names = {v: k for k, v in STAGE_VECTORS.items()}
         return {"stage_vectors": names[lc.stage_vectors], "modes_per_sm": int(lc.modes_per_sm),
                 "modes_in_flight": int(nf.value)}

@@ -207,6 +207,17 @@ int adj_upload_constants() {
 
 deb_internal::SmemLimit g_adj_smem;
 
+// Launch shape, by the items of the launch (not by the plan's room for them):
+// two blocks per SM (the registers' limit) when there are more items than SMs,
+// else one, each with the highest shared-memory level that leaves room.  ms with
+// one / two per SM on 152 SMs (likelihood gradients of one cosmology): nvar 323
+// 171 / 181 at 152 items, 166 / 173 at 153, 168 / 236 at 304, 166 / 229 at 400,
+// 247 / 249 at 608; nvar 1098 175 / 198, 174 / 197, 216 / 244, 253 / 253, 389 /
+// 308.  Two win where a launch has several items per SM; the line lies low, one
+// would still be as fast at up to 2.6.
+int adj_launch_blocks(const deb_plan* p, long items) { return (int)(items < p->adj_blocks ? items : p->adj_blocks); }
+int adj_two_per_sm(const deb_plan* p, int blocks) { return blocks > p->nsm ? 1 : 0; }
+
 }  // namespace
 
 extern "C" {
@@ -231,22 +242,21 @@ int deb_plan_create_adjoint(const deb_dims* dims, int max_items, int seg_cap, de
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
     return DEB_ERR_CUDA;
-  // Blocks per SM: two when there are items for them (the registers' limit),
-  // else one; the shared-memory level is the highest that leaves room for them.
   const deb::Dims Dm = deb::make_dims(dims->lmaxg, dims->lmaxgp, dims->lmaxr, dims->lmaxnu, dims->nqmax);
   const long fixed = (long)sizeof(deb::AdjS);
-  const int per_sm = max_items > nsm ? 2 : 1;
-  int level = 4;
-  for (; level > 0; --level) {
-    const long bytes = adj_smem_doubles(Dm, level) * (long)sizeof(double);
-    if (bytes + fixed <= optin && per_sm * (bytes + fixed + 1024) <= sm_bytes) break;
+  int level[2];
+  long smem[2];
+  for (int i = 0; i < 2; ++i) {
+    for (level[i] = 4; level[i] > 0; --level[i]) {
+      const long bytes = adj_smem_doubles(Dm, level[i]) * (long)sizeof(double);
+      if (bytes + fixed <= optin && (i + 1) * (bytes + fixed + 1024) <= sm_bytes) break;
+    }
+    smem[i] = adj_smem_doubles(Dm, level[i]) * (long)sizeof(double);
+    if (smem[i] + fixed > optin) return DEB_ERR_INVALID;
+    if (g_adj_smem.raise(adjoint_kernel, smem[i]) != cudaSuccess) return DEB_ERR_CUDA;
   }
-  const size_t smem = (size_t)adj_smem_doubles(Dm, level) * sizeof(double);
-  if (smem + fixed > (size_t)optin) return DEB_ERR_INVALID;
-  if (g_adj_smem.raise(adjoint_kernel, (long)smem) != cudaSuccess) return DEB_ERR_CUDA;
   deb_plan* p = new deb_plan();
-  p->adj_smem = (long)smem;
-  p->adj_level = level;
+  for (int i = 0; i < 2; ++i) { p->adj_smem[i] = smem[i]; p->adj_level[i] = level[i]; }
   p->D = deb::make_dims(dims->lmaxg, dims->lmaxgp, dims->lmaxr, dims->lmaxnu, dims->nqmax);
   p->nout = dims->nout;
   p->exec_mode = DEB_EXEC_WARP;
@@ -258,19 +268,29 @@ int deb_plan_create_adjoint(const deb_dims* dims, int max_items, int seg_cap, de
   p->adj_wslot = p->slot_len + (long)(deb::NAV + seg_cap) * p->D.n + kThetaLen + kSetLen;
   p->adj_wslot += p->adj_wslot & 1;
   // blocks in flight: what the SMs hold, capped by the items and by 32 GiB
-  long warps = (long)nsm * per_sm;
+  long blocks = (long)nsm * 2;
   const long mem_cap = (32L << 30) / (p->adj_wslot * 8);
-  if (warps > mem_cap) warps = mem_cap;
-  if (warps > max_items) warps = max_items;
-  if (warps < 1) { delete p; return DEB_ERR_NOMEM; }
-  p->adj_warps = (int)warps;
-  p->ws_bytes = (size_t)warps * p->adj_wslot * sizeof(double);
+  if (blocks > mem_cap) blocks = mem_cap;
+  if (blocks > max_items) blocks = max_items;
+  if (blocks < 1) { delete p; return DEB_ERR_NOMEM; }
+  p->adj_blocks = (int)blocks;
+  p->ws_bytes = (size_t)blocks * p->adj_wslot * sizeof(double);
   if (cudaMalloc(&p->adj_ws, p->ws_bytes) != cudaSuccess) { delete p; return DEB_ERR_NOMEM; }
   if (cudaMalloc(&p->queue, sizeof(int) * 4) != cudaSuccess) { cudaFree(p->adj_ws); delete p; return DEB_ERR_NOMEM; }
   if (cudaMalloc(&p->order_dev, sizeof(int) * (size_t)max_items) != cudaSuccess) {
     cudaFree(p->adj_ws); cudaFree(p->queue); delete p; return DEB_ERR_NOMEM;
   }
   *out = p;
+  return DEB_OK;
+}
+
+int deb_adjoint_launch_info(const deb_plan* p, int items, deb_launch_cfg* cfg, int* items_in_flight) {
+  if (!p || !p->adj || items < 1 || !cfg || !items_in_flight) return DEB_ERR_INVALID;
+  if (items > p->max_modes) return DEB_ERR_CAPACITY;
+  const int blocks = adj_launch_blocks(p, items), two = adj_two_per_sm(p, blocks), level = p->adj_level[two];
+  cfg->stage_vectors = level >= 2 ? DEB_STAGE_SHARED : level == 1 ? DEB_STAGE_GLOBAL : DEB_STAGE_ALL_GLOBAL;
+  cfg->modes_per_sm = 1 + two;
+  *items_in_flight = blocks;
   return DEB_OK;
 }
 
@@ -296,13 +316,13 @@ int deb_adjoint(deb_plan* p, const double* d_tables, const double* d_tables_pm, 
   P.ckpt = d_ckpt; P.ck_cap = ck_cap; P.ckoff = d_ckoff; P.ckstride = d_ckstride; P.gy = d_gy; P.gth = d_gtheta; P.status = d_status;
   P.ws = p->adj_ws; P.wslot = p->adj_wslot; P.seg_cap = p->adj_seg_cap; P.queue = p->queue; P.order = p->order_dev;
   P.D = p->D;
-  P.level = p->adj_level;
-  if (g_adj_smem.raise(adjoint_kernel, p->adj_smem) != cudaSuccess) return DEB_ERR_CUDA;
+  const long items = (long)nmode * nseed;
+  const int blocks = adj_launch_blocks(p, items), two = adj_two_per_sm(p, blocks);
+  P.level = p->adj_level[two];
+  if (g_adj_smem.raise(adjoint_kernel, p->adj_smem[two]) != cudaSuccess) return DEB_ERR_CUDA;
   if (cudaMemsetAsync(p->queue, 0, sizeof(int), s) != cudaSuccess) return DEB_ERR_CUDA;
   rank_desc_adj_kernel<<<(nmode + 255) / 256, 256, 0, s>>>(d_nrec, nmode, p->order_dev);
-  const long items = (long)nmode * nseed;
-  const int blocks = (int)(items < p->adj_warps ? items : p->adj_warps);
-  adjoint_kernel<<<blocks, kAdjThreads, (size_t)p->adj_smem, s>>>(P);
+  adjoint_kernel<<<blocks, kAdjThreads, (size_t)p->adj_smem[two], s>>>(P);
   return cudaGetLastError() == cudaSuccess ? DEB_OK : DEB_ERR_CUDA;
 }
 

@@ -29,12 +29,14 @@ struct deb_plan {
   const int* user_order;   // deb_plan_set_order
   int user_order_n;
   size_t ws_bytes;
-  // adjoint plans (deb_plan_create_adjoint): warps in flight, states per
-  // segment, per-warp workspace (doubles) and its array
-  int adj, adj_warps, adj_seg_cap;
+  // adjoint plans (deb_plan_create_adjoint): blocks in flight, states per
+  // segment, per-block workspace (doubles) and its array
+  int adj, adj_blocks, adj_seg_cap;
   long adj_wslot;
-  long adj_smem;   // dynamic shared memory of the adjoint launch (bytes)
-  int adj_level;   // what of an item's state lives in shared memory (deb_adjoint.cu)
+  // launch shape with one block per SM, with two: dynamic shared memory (bytes) and
+  // what of an item's state lives there (deb_adjoint.cu)
+  long adj_smem[2];
+  int adj_level[2];
   double* adj_ws;
 };
 

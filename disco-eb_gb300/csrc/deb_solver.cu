@@ -702,11 +702,7 @@ int deb_plan_create_grouped(const deb_dims* dims, int max_modes, int batch_size,
 int deb_plan_launch_info(const deb_plan* p, deb_launch_cfg* cfg, int* modes_in_flight) {
   if (!p || !cfg || !modes_in_flight) return DEB_ERR_INVALID;
   if (p->adj) {
-    // adjoint plan: warps (items) in flight and per SM; "shared" when its
-    // hottest vectors live in shared memory
-    cfg->stage_vectors = p->adj_level >= 2 ? DEB_STAGE_SHARED : p->adj_level == 1 ? DEB_STAGE_GLOBAL : DEB_STAGE_ALL_GLOBAL;
-    cfg->modes_per_sm = p->nsm > 0 ? (p->adj_warps + p->nsm - 1) / p->nsm : 0;
-    *modes_in_flight = p->adj_warps;
+    return deb_adjoint_launch_info(p, p->max_modes, cfg, modes_in_flight);
   } else if (p->group_size > 0) {
     cfg->stage_vectors = DEB_STAGE_GLOBAL;
     cfg->modes_per_sm = 0;

@@ -251,6 +251,11 @@ int deb_forward_record_ckpt(deb_plan* plan, const double* d_tables, int ncosmo, 
  * No counterpart in the reference (its gradient is forward mode).
  */
 int deb_plan_create_adjoint(const deb_dims* dims, int max_items, int seg_cap, deb_plan** plan);
+/* The shape a deb_adjoint launch of that many items (seeds times modes) takes on
+   the plan: where an item's state lives (shared: slot and stage vectors, global:
+   the slot alone, all_global: none of it), items per SM and in flight.
+   deb_plan_launch_info reports the shape at max_items. */
+int deb_adjoint_launch_info(const deb_plan* plan, int items, deb_launch_cfg* launch, int* items_in_flight);
 int deb_adjoint(deb_plan* plan, const double* d_tables, const double* d_tables_pm, int ncosmo, int npar, int blob_len,
                 const double* d_eps, const double* d_k, const int* d_cosmo_of_mode, int nmode,
                 const double* d_tau_out, const double* d_tau_out_pm, const double* d_record, int rec_len,
