@@ -18,8 +18,9 @@ struct deb_plan {
   int lane_blocks, lane_slots;
   // warp mode
   int block_warps, warp_blocks, warp_smem, warp_k_global, warp_per_sm;
-  // grouped plans (deb_plan_create_grouped): modes per group, warps in flight
-  int group_size, group_warps;
+  // grouped plans (deb_plan_create_grouped): modes per group, groups in flight
+  // with the slots in shared memory (0: they don't fit) and in global memory
+  int group_size, group_shared, group_global;
   long warp_smem_bytes;
   double* kws;      // warp mode: stage vectors in global memory
   double* ws;       // lane slots (or warp slots when shared memory is too small)

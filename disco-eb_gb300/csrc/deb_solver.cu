@@ -300,20 +300,31 @@ inline long block_static_bytes() { return (long)sizeof(deb::BlkS); }
 // groups of 16, where this takes 46.  A group whose modes are not all valid or
 // not all of one cosmology is marked BAD_INPUT.
 constexpr int kGroupWarps = 4;
+inline int group_warps(int batch_size) { return batch_size < kGroupWarps ? batch_size : kGroupWarps; }
+inline int group_blocks(int batch_size) { return (batch_size + group_warps(batch_size) - 1) / group_warps(batch_size); }
+// Slots in shared memory where all groups of the launch are in flight with them
+// there, or as many as the registers allow (eight warps per SM); else in global
+// memory.  nvar 323 (44 KB a slot, four or five per SM), groups of 1 / 4, shared
+// against global: 760 modes 32 / 30 ms against 33 / 30, 1216 37 / 36 against 37 /
+// 33, 2400 61 / 61 against 53 / 50; nvar 152 (22 KB), 2400 modes 39 / 41 against
+// 46 / 40.
+inline bool group_in_shared(const deb_plan* p, int ngroup) {
+  return p->group_shared >= ngroup || p->group_shared >= p->group_global;
+}
 
 __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams P, int B) {
   namespace cg = cooperative_groups;
   extern __shared__ double smem[];
   __shared__ double s_ss[2][kGroupWarps], s_t0[kGroupWarps];
   cg::cluster_group cluster = cg::this_cluster();
-  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, gw = blockDim.x >> 5;
   const int csize = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-  const int b = rank * kGroupWarps + wi;           // this warp's mode of a group (none for b >= B)
+  const int b = rank * gw + wi;                    // this warp's mode of a group (none for b >= B)
   const deb::Grp<32> gp{lane};
   const int osz = P.ctl.return_full ? P.D.n : DEB_NOUT_FIELDS;
   const int ngroup = P.nmode / B, nclust = (int)gridDim.x / csize, clust = (int)blockIdx.x / csize;
   // value of mode j of the group in array p of its block
-  auto of_mode = [&](double* p, int j) -> double { return *cluster.map_shared_rank(p + j % kGroupWarps, j / kGroupWarps); };
+  auto of_mode = [&](double* p, int j) -> double { return *cluster.map_shared_rank(p + j % gw, j / gw); };
   for (int q = clust; q < ngroup; q += nclust) {
     const int m0 = q * B, m = m0 + (b < B ? b : B - 1);
     const int ci = P.cosmo ? P.cosmo[m0] : 0;
@@ -336,8 +347,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
         deb::ModeCtx<32> x;
         x.c = c0;
         deb::mode_const(c0, P.k[m0 + j], x.m);
-        x.w.p = P.smem ? smem + (j % kGroupWarps) * P.slot_len
-                       : P.ws + ((long)clust * csize * kGroupWarps + j) * P.slot_len;
+        x.w.p = P.smem ? smem + (j % gw) * P.slot_len : P.ws + ((long)clust * csize * gw + j) * P.slot_len;
         x.w.n = P.D.n;
         x.w.misc0 = deb::V_K0 * P.D.n;
         x.w.kp = x.w.p + deb::hot_len(P.D);
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
         x.yout = P.y_out + (long)(m0 + j) * P.ctl.nout * osz;
         return x;
       };
-      const int step = csize * kGroupWarps;        // >= B: one pass of each loop below
+      const int step = csize * gw;                 // >= B: one pass of each loop below
       for (int j = b; j < B; j += step) {
         const deb::ModeCtx<32> x = ctx(j);
         const double ts = deb::mode_start(x.c, x.m, P.ctl, x.tau_out);
@@ -670,26 +680,34 @@ int deb_plan_create_grouped(const deb_dims* dims, int max_modes, int batch_size,
   p->slot_len = deb::slot_len(p->D);
   p->dense_len = 0;
   p->group_size = batch_size;
-  // a cluster of blocks of kGroupWarps warps per group; the slots in shared
-  // memory where a block's four fit, else in global memory
-  const int csize = (batch_size + kGroupWarps - 1) / kGroupWarps;
+  // a cluster of blocks of up to kGroupWarps warps per group; in flight what the
+  // registers (eight warps) or the slots leave room for on an SM, global slots up
+  // to 16 GiB; shared ones where those of four warps fit an SM
+  const int gw = group_warps(batch_size), csize = group_blocks(batch_size);
   const long groups = ((long)max_modes + batch_size - 1) / batch_size;
-  const long block_bytes = kGroupWarps * p->slot_len * (long)sizeof(double);
-  int optin = 0;
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) { delete p; return DEB_ERR_CUDA; }
-  p->warp_smem = block_bytes + 1024 <= optin ? 1 : 0;
-  p->warp_smem_bytes = p->warp_smem ? block_bytes : 0;
-  if (g_group_smem.raise(forward_group_kernel, p->warp_smem_bytes) != cudaSuccess) { delete p; return DEB_ERR_CUDA; }
-  // clusters in flight: two blocks per SM (registers), capped at 16 GiB of slots
-  long clusters = (long)nsm * 2 / csize;
-  if (!p->warp_smem) {
-    const long mem_cap = (16L << 30) / (block_bytes * csize);
-    if (clusters > mem_cap) clusters = mem_cap;
+  const long block_bytes = gw * p->slot_len * (long)sizeof(double);
+  int optin = 0, sm_bytes = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess) {
+    delete p;
+    return DEB_ERR_CUDA;
   }
-  if (clusters > groups) clusters = groups;
-  if (clusters < 1) clusters = 1;
-  p->group_warps = (int)clusters;
-  p->ws_bytes = p->warp_smem ? 0 : (size_t)clusters * csize * block_bytes;
+  auto in_flight = [&](long blocks_per_sm) {
+    const long c = nsm * blocks_per_sm / csize;
+    return c > 1 ? c : 1;
+  };
+  long shared = 0, global = in_flight(8 / gw);
+  if (kGroupWarps * p->slot_len * (long)sizeof(double) + 1024 <= optin) {
+    const long by_smem = sm_bytes / (block_bytes + 1024);
+    shared = in_flight(by_smem < 8 / gw ? by_smem : 8 / gw);
+    if (g_group_smem.raise(forward_group_kernel, block_bytes) != cudaSuccess) { delete p; return DEB_ERR_CUDA; }
+  }
+  const long mem_cap = (16L << 30) / (block_bytes * csize);
+  if (mem_cap >= 1 && global > mem_cap) global = mem_cap;
+  p->group_shared = (int)shared;
+  p->group_global = (int)global;
+  p->warp_smem_bytes = block_bytes;
+  p->ws_bytes = group_in_shared(p, (int)groups) ? 0 : (size_t)(global < groups ? global : groups) * csize * block_bytes;
   if (p->ws_bytes && cudaMalloc(&p->ws, p->ws_bytes) != cudaSuccess) { delete p; return DEB_ERR_NOMEM; }
   if (cudaMalloc(&p->queue, sizeof(int) * 4) != cudaSuccess) { cudaFree(p->ws); delete p; return DEB_ERR_NOMEM; }
   if (cudaMalloc(&p->order_dev, sizeof(int)) != cudaSuccess) {
@@ -704,9 +722,11 @@ int deb_plan_launch_info(const deb_plan* p, deb_launch_cfg* cfg, int* modes_in_f
   if (p->adj) {
     return deb_adjoint_launch_info(p, p->max_modes, cfg, modes_in_flight);
   } else if (p->group_size > 0) {
-    cfg->stage_vectors = DEB_STAGE_GLOBAL;
+    const int groups = (int)(((long)p->max_modes + p->group_size - 1) / p->group_size);
+    const int room = group_in_shared(p, groups) ? p->group_shared : p->group_global;
+    cfg->stage_vectors = group_in_shared(p, groups) ? DEB_STAGE_SHARED : DEB_STAGE_ALL_GLOBAL;
     cfg->modes_per_sm = 0;
-    *modes_in_flight = p->group_warps * p->group_size;
+    *modes_in_flight = (groups < room ? groups : room) * p->group_size;
   } else if (p->exec_mode == DEB_EXEC_LANE) {
     cfg->stage_vectors = DEB_STAGE_GLOBAL;
     cfg->modes_per_sm = 0;
@@ -831,13 +851,13 @@ int deb_forward_grouped(deb_plan* p, const double* d_tables, int ncosmo, int blo
   P.ctl.max_steps = cfg->max_steps; P.ctl.hist_on_reject = cfg->hist_on_reject;
   P.ctl.dense = 0; P.ctl.return_full = 0; P.ctl.nout = p->nout;
   P.ctl.record = 0; P.ctl.replay = 0; P.ctl.step_ts = 0;
-  P.smem = p->warp_smem;
-  const int ngroup = nmode / p->group_size, csize = (p->group_size + kGroupWarps - 1) / kGroupWarps;
-  const int clusters = ngroup < p->group_warps ? ngroup : p->group_warps;
+  const int ngroup = nmode / p->group_size, gw = group_warps(p->group_size), csize = group_blocks(p->group_size);
+  P.smem = group_in_shared(p, ngroup);
+  const int room = P.smem ? p->group_shared : p->group_global, clusters = ngroup < room ? ngroup : room;
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3((unsigned)(clusters * csize));
-  lc.blockDim = dim3(32 * kGroupWarps);
-  lc.dynamicSmemBytes = (size_t)p->warp_smem_bytes;
+  lc.blockDim = dim3(32 * (unsigned)gw);
+  lc.dynamicSmemBytes = P.smem ? (size_t)p->warp_smem_bytes : 0;
   lc.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
