@@ -288,10 +288,11 @@ struct WS {
 };
 
 // A group of G lanes that cooperates on one mode: G = 1 (one thread per
-// mode; also the host build) or G = 32 (one warp per mode, state in shared
-// memory).  Vector loops stride by G, chains are spread over lanes, scalar
-// work is done redundantly or by the leading lane.  No sync/shuffle may sit
-// inside a lane-divergent branch.
+// mode; also the host build), G = 32 (one warp per mode, state in shared
+// memory) or a whole block of more (deb_block.cuh; loops and barriers only).
+// Vector loops stride by G, chains are spread over lanes, scalar work is done
+// redundantly or by the leading lane.  No sync/shuffle may sit inside a
+// lane-divergent branch.
 template <int G>
 struct Grp {
   int lane;
@@ -303,6 +304,7 @@ struct Grp {
 #endif
   }
   HD double sum(double x) const {
+    static_assert(G <= 32, "shuffles reach one warp");
 #ifdef __CUDA_ARCH__
     if (G > 1)
       for (int o = G / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -315,6 +317,7 @@ struct Grp {
   // split the values over half- and quarter-warps: 5 adds for two sums and
   // 6 for three instead of 10 and 15.
   HD void sum2(double& a, double& b) const {
+    static_assert(G <= 32, "shuffles reach one warp");
 #ifdef __CUDA_ARCH__
     if (G == 32) {
       const bool lo = lane < 16;
@@ -329,6 +332,7 @@ struct Grp {
     b = sum(b);
   }
   HD void sum3(double& a, double& b, double& c) const {
+    static_assert(G <= 32, "shuffles reach one warp");
 #ifdef __CUDA_ARCH__
     if (G == 32) {
       const bool lo = lane < 16, q = (lane & 8) == 0;
@@ -347,6 +351,7 @@ struct Grp {
     c = sum(c);
   }
   HD double bcast(double x, int src) const {
+    static_assert(G <= 32, "shuffles reach one warp");
 #ifdef __CUDA_ARCH__
     if (G > 1) return __shfl_sync(0xffffffffu, x, src);
 #endif
@@ -354,6 +359,7 @@ struct Grp {
   }
   HD Dual bcast(Dual x, int src) const { return Dual(bcast(x.v, src), bcast(x.d, src)); }
   HD bool any(bool b) const {
+    static_assert(G <= 32, "shuffles reach one warp");
 #ifdef __CUDA_ARCH__
     if (G > 1) return __any_sync(0xffffffffu, b);
 #endif
@@ -361,6 +367,7 @@ struct Grp {
   }
   // index of the largest |value| (first index on ties) across the group
   HD void argmax(double& best, int& bi) const {
+    static_assert(G <= 32, "shuffles reach one warp");
 #ifdef __CUDA_ARCH__
     if (G > 1)
       for (int o = G / 2; o > 0; o >>= 1) {
