@@ -727,8 +727,8 @@ def run_loglike(args, inp, world, rank, local):
                           "the timed call) and the data vector; P(k, a), ln L and the gradient copied back"},
         "roofline": {"bound": "fp64", "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
                      "frac": achieved / peak, "traffic": ADJ_DRAM_BYTES_PER_STEP * acc, "kernel": "adjoint_kernel",
-                     "note": "FP64 pipe ~half busy, latency-bound (2 warps per scheduler at 255 registers, global-memory "
-                             "waits); peak = FP64 FMA microkernel measured in this run (MEASURED_PEAKS.json has no FP64 "
+                     "note": "FP64 pipe 39 to 41 % busy in a captured adjoint, over a third of a warp's time at barriers "
+                             "(2 warps per scheduler at 254 registers); peak = FP64 FMA microkernel measured in this run (MEASURED_PEAKS.json has no FP64 "
                              "figure); achieved = algorithmic FLOPs of the adjoint sweep (per accepted step + "
                              "recomputed segment steps) / the adjoint launch's time; traffic = DRAM bytes per accepted "
                              "step of an ncu capture of the counter-capture workload x accepted steps"},

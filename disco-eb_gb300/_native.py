@@ -42,7 +42,8 @@ EXPORTS = ("deb_nvar", "deb_plan_create", "deb_plan_create_ex", "deb_plan_launch
            "deb_plan_set_order", "deb_forward", "deb_forward_static", "deb_tables_blob_len", "deb_evolve_background",
            "deb_evolve_background_host", "deb_evolve_background_frozen", "deb_evolve_background_frozen_host",
            "deb_tau_of_a", "deb_plan_create_grouped", "deb_forward_grouped",
-           "deb_forward_record", "deb_forward_record_ckpt", "deb_plan_create_adjoint", "deb_adjoint_launch_info", "deb_adjoint", "deb_replay",
+           "deb_forward_record", "deb_forward_record_ckpt", "deb_plan_create_adjoint", "deb_adjoint_launch_info",
+           "deb_adjoint", "deb_replay",
            "deb_get_power", "deb_power_multipoles", "deb_density_velocity",
            "deb_power_kaiser", "deb_savgol_log", "deb_fftlog_phase",
            "deb_plan_destroy", "deb_measure_fp64_peak", "deb_error_string", "deb_version")

@@ -77,7 +77,7 @@ long adj_smem_doubles(const deb::Dims& D, int level) {
 // Two blocks per SM at 254 registers: eight warps of FP64 work hide each
 // other's latencies, and a register limit for more spills.  Measured against
 // one warp per item (one likelihood gradient from Python): nvar 323, 128 k, 8
-// outputs: 948 -> 247 ms; nvar 1098, 96 k, 64 outputs: 837 -> 227 ms.
+// outputs: 935 -> 229 ms; nvar 1098, 96 k, 64 outputs: 799 -> 230 ms.
 __global__ void __launch_bounds__(kAdjThreads, 2) adjoint_kernel(AParams P) {
   extern __shared__ double smem[];
   __shared__ __align__(16) unsigned char raw[sizeof(deb::AdjS)];   // no constructor runs

@@ -1,8 +1,11 @@
 // deb_adjoint.cuh -- discrete adjoint (reverse mode) of the Rodas5 solve of
 // one k-mode on its recorded step sequence: d L / d theta for a cotangent of
-// the 20 output fields at every output time.  Host/device code like
-// deb_core.cuh: the CUDA kernel splits it over a block per (seed, mode) item
-// (deb_adjoint_block.cuh), the test suite compiles it for the host.
+// the 20 output fields at every output time.  The whole of it runs on the host,
+// where the test suite checks the mathematics against dense Jacobians and
+// difference quotients.  The CUDA kernel takes the coefficients, the lead rows'
+// lists, the output conversion's adjoint, the item and its times from here and
+// splits the rest over a block per (seed, mode) item in its own form
+// (deb_adjoint_block.cuh), checked on the GPU against replayed quotients.
 //
 // What is differentiated.  The reference differentiates its solve with
 // jax.jacfwd (perturbations.py:765, DirectAdjoint; compute_matter_power in

@@ -536,7 +536,6 @@ struct AdjBlk {
 
   // the remaining entries of a form from its sums (one warp)
   __device__ void assemble(const double* Y, int f, double* B, bool add) {
-    const int n = D.n, ir = D.ir;
     const double xh1 = S.xk[DK_HP1] + 0.5 * S.xk[DK_ALPHA] + S.hn, xhw = S.xk[DK_HPW];
     const double xe = S.xk[DK_E] + 3.0 * S.xk[DK_ALPHA] + S.en, xp = S.xk[DK_P1];
     for (int e = lane; e < NB - NSIG; e += 32) {
@@ -562,7 +561,6 @@ struct AdjBlk {
       }
       B[j] = add ? B[j] + v : v;
     }
-    (void)n; (void)ir;
     __syncwarp();
   }
   // the fixed elements the functionals read: h' (0), eta' (1), P1 (2)
@@ -583,7 +581,7 @@ struct AdjBlk {
     const Coef<double>& C = *reinterpret_cast<const Coef<double>*>(Cv);
     const Coef<double>& E = *reinterpret_cast<const Coef<double>*>(C1v);
     const LeadLists& Q = S.lead;
-    const int n = D.n, nq = D.nq, iq0 = D.iq0, ir = D.ir;
+    const int nq = D.nq, iq0 = D.iq0;
     for (int sl = lane; sl < Q.nslot; sl += 32) {
       double s = 0.0;
       for (int e = Q.slot_at[sl]; e < Q.slot_at[sl + 1]; ++e)
@@ -626,7 +624,6 @@ struct AdjBlk {
       z[iq0 + i] += s;
       z[iq0 + nq + i] += e;
     }
-    (void)n; (void)ir;
     __syncwarp();
   }
 

@@ -1,7 +1,8 @@
 // deb_block.cuh -- one Rodas5 step of one k-mode by a thread block (device
 // only; structured solver).  Same arithmetic as step_attempt of deb_core.cuh,
-// operation by operation, so both give the same bits; what differs is which
-// thread evaluates which expression.
+// operation by operation, so both take the same steps; what differs is which
+// thread evaluates which expression.  (Output fields agree to 1e-15: their
+// conversion is compiled separately in the two kernels.)
 //
 // What bounds a step.  GB300 issues one FP64 instruction per 64 cycles to a
 // warp, however many of its lanes are active, and one per ~19 cycles to an SM

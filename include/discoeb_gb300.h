@@ -74,7 +74,8 @@ enum deb_exec_mode {
   DEB_EXEC_AUTO = 0,        /* block or warp per mode for small batches, lane per mode for large ones */
   DEB_EXEC_LANE = 1,        /* one thread per mode, state interleaved in global memory */
   DEB_EXEC_WARP = 2         /* a block of four warps (structured solver, nqmax <= 32) or one warp per mode,
-                               state in shared memory */
+                               state in shared memory; one warp too where DEB_STAGE_SHARED is asked for and
+                               a mode's slot fits only without the block's own share */
 };
 
 /* hierarchy sizes: the keyword arguments of evolve_perturbations (perturbations.py:926-930) */
