@@ -312,20 +312,20 @@ inline bool group_in_shared(const deb_plan* p, int ngroup) {
   return p->group_shared >= ngroup || p->group_shared >= p->group_global;
 }
 
-__global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams P, int B) {
+__global__ void __launch_bounds__(32 * kGroupWarps, 2) forward_group_kernel(KParams P, int B) {
   namespace cg = cooperative_groups;
   extern __shared__ double smem[];
   __shared__ double s_ss[2][kGroupWarps], s_t0[kGroupWarps];
-  __shared__ int s_q[2];
+  __shared__ int s_q;
   cg::cluster_group cluster = cg::this_cluster();
-  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, gw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const int csize = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-  const int b = rank * gw + wi;                    // this warp's mode of a group (none for b >= B)
+  const int b = rank * ((int)blockDim.x >> 5) + wi;   // this warp's mode of a group (none for b >= B)
   const deb::Grp<32> gp{lane};
   const int osz = P.ctl.return_full ? P.D.n : DEB_NOUT_FIELDS;
-  const int ngroup = P.nmode / B, nclust = (int)gridDim.x / csize, clust = (int)blockIdx.x / csize;
-  // value of mode j of the group in array p of its block
-  auto of_mode = [&](double* p, int j) -> double { return *cluster.map_shared_rank(p + j % gw, j / gw); };
+  const int ngroup = P.nmode / B;
+  // value of mode j of the group in array p of its block (blocks of kGroupWarps, or one)
+  auto of_mode = [&](double* p, int j) -> double { return *cluster.map_shared_rank(p + j % kGroupWarps, j / kGroupWarps); };
   // A cluster begins with a group of its own and takes further ones from a
   // queue, the last group first (k-grids ascend, and the lowest k take the fewest
   // steps): step counts differ several times over, and dealt out by a stride one
@@ -334,8 +334,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
   // groups of 16 241 / 120.  The first groups by index, so that neighbours in k
   // (of similar cost) do not share an SM: 1200 modes of nvar 492 in groups of 4,
   // all in flight, 42 ms, with a queue from the start 51.
-  int q = ngroup - 1 - clust;
-  for (int turn = 0; q >= 0; turn ^= 1) {
+  int q = ngroup - 1 - (int)blockIdx.x / csize;
+  while (q >= 0) {
     const int m0 = q * B, m = m0 + (b < B ? b : B - 1);
     const int ci = P.cosmo ? P.cosmo[m0] : 0;
     bool ok = ci >= 0 && ci < P.ncosmo;
@@ -353,22 +353,21 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
     run.rec = nullptr; run.rec_cap = 0; run.nrec = 0; run.acc = 0; run.rej = 0; run.status = deb::ST_BAD_INPUT;
     if (ok) {                                      // the same for every warp of the cluster
       const double* tau_out = P.tau_out + (long)ci * P.ctl.nout;
-      auto ctx = [&](int j) {
+      auto ctx = [&]() {                           // this warp's mode
         deb::ModeCtx<32> x;
         x.c = c0;
-        deb::mode_const(c0, P.k[m0 + j], x.m);
-        x.w.p = P.smem ? smem + (j % gw) * P.slot_len : P.ws + ((long)clust * csize * gw + j) * P.slot_len;
+        deb::mode_const(c0, P.k[m], x.m);
+        x.w.p = P.smem ? smem + wi * P.slot_len : P.ws + (long)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * P.slot_len;
         x.w.n = P.D.n;
         x.w.misc0 = deb::V_K0 * P.D.n;
         x.w.kp = x.w.p + deb::hot_len(P.D);
         x.w.dp = nullptr;
         x.tau_out = tau_out;
-        x.yout = P.y_out + (long)(m0 + j) * P.ctl.nout * osz;
+        x.yout = P.y_out + (long)m * P.ctl.nout * osz;
         return x;
       };
-      const int step = csize * gw;                 // >= B: one pass of each loop below
-      for (int j = b; j < B; j += step) {
-        const deb::ModeCtx<32> x = ctx(j);
+      if (b < B) {
+        const deb::ModeCtx<32> x = ctx();
         const double ts = deb::mode_start(x.c, x.m, P.ctl, x.tau_out);
         if (lane == 0) s_t0[wi] = ts;
       }
@@ -376,8 +375,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
       double t0 = 1e300;
       for (int j = 0; j < B; ++j) { const double ts = of_mode(s_t0, j); t0 = ts < t0 ? ts : t0; }
       run.t0 = 0.0; run.T1 = 0.0; run.status = deb::ST_OK;
-      for (int j = b; j < B; j += step) {
-        const deb::ModeCtx<32> x = ctx(j);
+      if (b < B) {
+        const deb::ModeCtx<32> x = ctx();
         deb::mode_begin<32>(gp, x.c, x.m, P.D, P.ctl, x.w, x.tau_out, run, t0);
       }
       // the modes' run.t0, T1 and steps are the group's, so all end together;
@@ -387,11 +386,10 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
         if (go && run.steps >= P.ctl.max_steps) { run.status = deb::ST_MAX_STEPS; go = false; }
         bool bad = false;
         double ss = -1.0;
-        if (go)
-          for (int j = b; j < B; j += step) {
-            const deb::ModeCtx<32> x = ctx(j);
-            ss = deb::step_attempt<32>(gp, x.c, x.m, P.D, c_tab, c_rodas, P.ctl, x.w, run, bad);
-          }
+        if (go && b < B) {
+          const deb::ModeCtx<32> x = ctx();
+          ss = deb::step_attempt<32>(gp, x.c, x.m, P.D, c_tab, c_rodas, P.ctl, x.w, run, bad);
+        }
         if (b < B && lane == 0) s_ss[it & 1][wi] = ss;
         cluster.sync();
         if (of_mode(s_ss[it & 1], 0) < 0.0) break;
@@ -399,8 +397,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
         for (int j = 0; j < B; ++j) sum += of_mode(s_ss[it & 1], j);
         const double err = sqrt(sum / (6.0 * B));
         bool more = true;
-        for (int j = b; j < B; j += step) {
-          const deb::ModeCtx<32> x = ctx(j);
+        if (b < B) {
+          const deb::ModeCtx<32> x = ctx();
           more = deb::step_decide<32>(gp, x.c, x.m, P.D, P.ctl, x.w, x.tau_out, x.yout, 1, run, err, bad);
         }
         if (!more) run.T1 = run.t0;
@@ -411,11 +409,21 @@ __global__ void __launch_bounds__(32 * kGroupWarps) forward_group_kernel(KParams
       P.status[m] = run.status;
       if (P.steps) { P.steps[2 * m] = run.acc; P.steps[2 * m + 1] = run.rej; }
     }
-    if (rank == 0 && threadIdx.x == 0) s_q[turn] = nclust + atomicAdd(P.queue, 1);
+    if (rank == 0 && threadIdx.x == 0) s_q = (int)gridDim.x / csize + atomicAdd(P.queue, 1);
     cluster.sync();
-    q = ngroup - 1 - *cluster.map_shared_rank(s_q + turn, 0);
+    q = ngroup - 1 - *cluster.map_shared_rank(&s_q, 0);
+    cluster.sync();                                // the first block's queue word is not read any more
   }
-  cluster.sync();                                  // the first block's queue word is not read any more
+  // The last cluster leaves the counters at zero for the next launch: a reset of
+  // its own before each launch could come between another thread's reset and
+  // kernel on the same stream.
+  if (rank == 0 && threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(P.queue + 1, 1) == (int)gridDim.x / csize - 1) {
+      P.queue[0] = 0;
+      P.queue[1] = 0;
+    }
+  }
 }
 
 __global__ void power_kernel(const double* tables, int ncosmo, int blob_len, const double* k, const int* cosmo, int nmode,
@@ -722,7 +730,11 @@ int deb_plan_create_grouped(const deb_dims* dims, int max_modes, int batch_size,
   p->warp_smem_bytes = block_bytes;
   p->ws_bytes = group_in_shared(p, (int)groups) ? 0 : (size_t)(global < groups ? global : groups) * csize * block_bytes;
   if (p->ws_bytes && cudaMalloc(&p->ws, p->ws_bytes) != cudaSuccess) { delete p; return DEB_ERR_NOMEM; }
-  if (cudaMalloc(&p->queue, sizeof(int)) != cudaSuccess) { cudaFree(p->ws); delete p; return DEB_ERR_NOMEM; }
+  // counters of the groups taken and of the clusters done, zero between launches
+  if (cudaMalloc(&p->queue, sizeof(int) * 2) != cudaSuccess) { cudaFree(p->ws); delete p; return DEB_ERR_NOMEM; }
+  if (cudaMemset(p->queue, 0, sizeof(int) * 2) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    cudaFree(p->ws); cudaFree(p->queue); delete p; return DEB_ERR_CUDA;
+  }
   *out = p;
   return DEB_OK;
 }
@@ -863,7 +875,6 @@ int deb_forward_grouped(deb_plan* p, const double* d_tables, int ncosmo, int blo
   P.ctl.record = 0; P.ctl.replay = 0; P.ctl.step_ts = 0;
   const int ngroup = nmode / p->group_size, gw = group_warps(p->group_size), csize = group_blocks(p->group_size);
   P.smem = group_in_shared(p, ngroup);
-  if (cudaMemsetAsync(p->queue, 0, sizeof(int), s) != cudaSuccess) return DEB_ERR_CUDA;
   const int room = P.smem ? p->group_shared : p->group_global, clusters = ngroup < room ? ngroup : room;
   cudaLaunchConfig_t lc{};
   lc.gridDim = dim3((unsigned)(clusters * csize));

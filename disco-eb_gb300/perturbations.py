@@ -292,7 +292,8 @@ def solve_grouped(tables, kmodes, tau_out, batch_size: int, cosmo_of_mode=None, 
         raise ValueError("the number of modes must be divisible by batch_size")
     com = as_t(np.zeros(nmode, dtype=np.int32) if cosmo_of_mode is None else cosmo_of_mode, torch.int32)
     dims = _dims(lmaxg, lmaxgp, lmaxr, lmaxnu, nqmax, nout, False, "structured", "warp")
-    key = ("grouped", torch.cuda.current_device(), lmaxg, lmaxgp, lmaxr, lmaxnu, nqmax, nout, int(batch_size))
+    stream = torch.cuda.current_stream().cuda_stream     # a plan's counters and slots serve one stream
+    key = ("grouped", torch.cuda.current_device(), lmaxg, lmaxgp, lmaxr, lmaxnu, nqmax, nout, int(batch_size), stream)
     plan = _plans.get(key)
     if plan is None or plan.max_modes < nmode:
         plan = _native.Plan(dims, max(nmode, 1), batch_size=int(batch_size))
@@ -304,7 +305,7 @@ def solve_grouped(tables, kmodes, tau_out, batch_size: int, cosmo_of_mode=None, 
     c = lambda t: ctypes.c_void_p(t.data_ptr())
     _native.check(_native.load().deb_forward_grouped(plan.ptr, c(tabs), int(tabs.shape[0]), int(tabs.shape[1]), c(k),
                                                      c(com), nmode, c(tau), ctypes.byref(cfg), c(y), c(status), c(steps),
-                                                     ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)),
+                                                     ctypes.c_void_p(stream)),
                   "deb_forward_grouped")
     st = status.cpu().numpy()
     _check_status(st, k.cpu().numpy(), throw)
